@@ -1946,6 +1946,8 @@ struct RunBufs {
     int32_t* status;
     int32_t* error;
     double* partials;
+    double* theta;        // [m][b] nodes and first eigenvector entries
+    double* tau;
     double* samples;
     double* params;
     uint64_t* starts;
@@ -2054,6 +2056,8 @@ void carve(Carver& c, const RunPlan& r, int sms, RunBufs* B)
     const size_t pcols = std::max<size_t>(static_cast<size_t>(sms) * 4 * r.b,
                                           static_cast<size_t>(sms) * 2 * MAX_J * r.b);
     B->partials = c.take<double>(pcols);
+    B->theta = c.take<double>(static_cast<size_t>(r.m) * r.b);
+    B->tau = c.take<double>(static_cast<size_t>(r.m) * r.b);
     B->samples = c.take<double>(static_cast<size_t>(r.b) * r.q);
     B->params = c.take<double>(r.q);
     B->starts = c.take<uint64_t>(static_cast<size_t>(r.b) * 4);
@@ -2078,6 +2082,25 @@ slq_status launch_probes(Launcher& L, const RunPlan& r, int rng, int64_t seed, i
         k_probe_fast<VT><<<grid, 128, 0, L.st>>>(r.nv, r.b, count, first,
                                                  static_cast<uint64_t>(seed) * 0xd1342543de82ef95ULL,
                                                  r.wpp, r.cw, inv, X);
+    SLQ_LAUNCH_CK();
+    ++L.launches;
+    return SLQ_OK;
+}
+
+// Nodes, weights and samples of a finished block's first `count` probes.
+slq_status launch_quadrature(Launcher& L, const RunPlan& r, const slq_params* p, const RunBufs& B,
+                             int count, double* samples, int32_t* status)
+{
+    ProfScope prof(SLQ_K_EIG, double(r.m) * r.b * 16.0 + double(count) * r.q * 8.0, L.st);
+    k_ql<<<count, 32, 3 * sizeof(double) * r.m, L.st>>>(r.b, r.m, B.alpha, B.beta, B.size,
+                                                        r.gram == 1, B.theta, B.tau, status);
+    SLQ_LAUNCH_CK();
+    ++L.launches;
+    const int64_t pairs = int64_t(count) * r.q;
+    const int grid = static_cast<int>(std::min<int64_t>((pairs + 7) / 8, int64_t(L.sms) * 8));
+    k_quad<<<grid, 256, 0, L.st>>>(count, r.b, r.m, B.size, B.theta, B.tau, p->func,
+                                   func_coeff(p), p->exponent, B.params, r.q,
+                                   static_cast<double>(r.nv), samples, status);
     SLQ_LAUNCH_CK();
     ++L.launches;
     return SLQ_OK;
@@ -2421,15 +2444,7 @@ slq_status run_typed(slq_op* op, const slq_params* p, const double* parameters, 
         ++L.launches;
         }
         SLQ_TRY(krylov_block<VT>(L, op, p, r, B, count, shift));
-        {
-        ProfScope prof(SLQ_K_EIG, double(m) * b * 16.0 + double(count) * q * 8.0, st);
-        k_eig_quad<<<(count + 127) / 128, 128, 0, st>>>(
-            count, b, m, B.alpha, B.beta, B.size, r.gram == 1, p->func, func_coeff(p),
-            p->exponent, B.params, q, static_cast<double>(r.nv), B.samples, nullptr, nullptr,
-            B.status);
-        SLQ_LAUNCH_CK();
-        ++L.launches;
-        }
+        SLQ_TRY(launch_quadrature(L, r, p, B, count, B.samples, B.status));
         SLQ_CK(cudaMemcpyAsync(hs.data(), B.samples, sizeof(double) * count * q,
                                cudaMemcpyDeviceToHost, st));
         SLQ_CK(cudaMemcpyAsync(hsize.data(), B.size, sizeof(int32_t) * count,
@@ -2806,12 +2821,8 @@ slq_status batch_enqueue(BatchRun& R, cudaStream_t st, int sms)
         SLQ_LAUNCH_CK();
         ++L.launches;
         SLQ_TRY(krylov_block<VT>(L, R.op, p, r, B, count, R.shift));
-        k_eig_quad<<<(count + 127) / 128, 128, 0, st>>>(
-            count, r.b, r.m, B.alpha, B.beta, B.size, r.gram == 1, p->func, func_coeff(p),
-            p->exponent, B.params, r.q, static_cast<double>(r.nv), R.samples + static_cast<size_t>(g) * r.q,
-            nullptr, nullptr, R.status + g);
-        SLQ_LAUNCH_CK();
-        ++L.launches;
+        SLQ_TRY(launch_quadrature(L, r, p, B, count, R.samples + static_cast<size_t>(g) * r.q,
+                                  R.status + g));
         const size_t ab = static_cast<size_t>(r.m) * r.b;
         SLQ_CK(cudaMemcpyAsync(R.size + g, B.size, sizeof(int32_t) * count,
                                cudaMemcpyDeviceToDevice, st));
@@ -3699,9 +3710,8 @@ extern "C" slq_status slq_nodes_weights(const double* alpha, const double* beta,
         m > EIG_MAX)
         return fail(SLQ_ERR_BAD_ARG, "nodes_weights: bad argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    k_eig_quad<<<(count + 127) / 128, 128, 0, st>>>(count, count, m, alpha, beta, sizes, gram, 0,
-                                                   make_double4(0.0, 0.0, 0.0, 0.0), 1.0, nullptr,
-                                                   0, 1.0, nullptr, theta, tau, status);
+    k_ql<<<count, 32, 3 * sizeof(double) * m, st>>>(count, m, alpha, beta, sizes, gram, theta, tau,
+                                                    status);
     SLQ_LAUNCH_CK();
     return SLQ_OK;
 }
