@@ -1107,96 +1107,123 @@ struct Launcher {
     int64_t launches = 0;
 };
 
-template <typename VT, int LV, int KS>
-slq_status spmm_inst(Launcher& L, int grid, const int32_t* ptr, const int32_t* ind,
-                     const VT* vals, int64_t nrows, int b, const VT* X,
-                     const double* sx, double shift, VT* Y, const VT* Z,
-                     const double* zc, const double* zs, int epi, double* partials,
-                     int64_t nnz, int64_t xrows)
+// compulsory traffic of a product: matrix once, X once, Y written once, Z
+// read once
+template <typename VT>
+double spmm_bytes(int64_t nnz, int64_t nrows, int64_t xrows, int b, bool z)
 {
-    // compulsory traffic: matrix once, X once, Y written once, Z read once
     const double s = sizeof(VT);
-    const double bytes = nnz * (s + 4.0) + (nrows + 1) * 4.0 + double(xrows) * b * s +
-                         double(nrows) * b * s * (Z ? 2.0 : 1.0);
-    ProfScope prof(SLQ_K_SPMM, bytes, L.st);
-    static bool attr = false;
+    return nnz * (s + 4.0) + (nrows + 1) * 4.0 + double(xrows) * b * s +
+           double(nrows) * b * s * (z ? 2.0 : 1.0);
+}
+
+template <typename VT, int LV, int KS>
+slq_status spmm_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, const VT* vals,
+                     int64_t nrows, int b, const VT* X, const double* sx, double shift, VT* Y,
+                     const VT* Z, const double* zc, const double* zs, int epi, double* partials,
+                     int64_t nnz, int64_t xrows, int* grid_out)
+{
+    ProfScope prof(SLQ_K_SPMM, spmm_bytes<VT>(nnz, nrows, xrows, b, Z != nullptr), L.st);
     const size_t smem = (epi != 0) ? 8 * static_cast<size_t>(b) * sizeof(double) : 0;
-    if (!attr)
-    {
-        SLQ_CK(cudaFuncSetAttribute(k_spmm<VT, LV, KS>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        attr = true;
-    }
+    const int grid = static_cast<int>(
+        std::max<int64_t>(1, std::min<int64_t>((nrows + 7) / 8, int64_t(L.sms) * 4)));
     k_spmm<VT, LV, KS><<<grid, 256, smem, L.st>>>(ptr, ind, vals, nrows, b, X, sx, shift, Y, Z,
                                                   zc, zs, epi, partials);
     SLQ_LAUNCH_CK();
     ++L.launches;
+    *grid_out = grid;
     return SLQ_OK;
 }
 
-// blocks of k_spmm<VT, LV, KS> resident per SM (occupancy query, at most 4)
-template <typename VT, int LV, int KS>
-int spmm_blocks_per_sm(int b)
+// k_spmm_rows: a persistent grid of the blocks that are resident at once (a
+// partial second wave would leave SMs idle at the end), at most 4 per SM (the
+// partial-sum buffer's rows); matrices with fewer rows than the SMs have
+// warps take smaller blocks, so that every SM gets some.
+template <typename VT, int LPR, int C, bool PLAIN>
+slq_status spmm_rows_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, const VT* vals,
+                          int64_t nrows, const VT* X, const double* sx, double shift, VT* Y,
+                          const VT* Z, const double* zc, const double* zs, int epi,
+                          double* partials, int64_t nnz, int64_t xrows, int* grid_out)
 {
-    static int cached = 0;
-    if (cached == 0)
+    constexpr int RW = 32 / LPR;
+    constexpr int b = LPR * C * (16 / static_cast<int>(sizeof(VT)));
+    ProfScope prof(SLQ_K_SPMM, spmm_bytes<VT>(nnz, nrows, xrows, b, Z != nullptr), L.st);
+    auto smem_of = [&](int warps) { return static_cast<size_t>(warps) * RW * b * sizeof(double); };
+    if (smem_of(8) > 48 * 1024)
+        SLQ_CK(cudaFuncSetAttribute(k_spmm_rows<VT, LPR, C, PLAIN>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem_of(8))));
+    static std::atomic<int> resident{0};
+    int per_sm = resident.load();
+    if (per_sm == 0)
     {
         int v = 0;
-        const size_t smem = 8 * static_cast<size_t>(b) * sizeof(double);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_spmm<VT, LV, KS>, 256, smem) !=
-                cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_spmm_rows<VT, LPR, C, PLAIN>, 256,
+                                                          smem_of(8)) != cudaSuccess ||
             v < 1)
             v = 1;
-        cached = std::min(v, 4);
+        per_sm = std::min(v, 4);
+        resident.store(per_sm);
     }
-    return cached;
+    int warps = 8;
+    while (warps > 1 && nrows <= int64_t(L.sms) * RW * warps / 2) warps >>= 1;
+    const int64_t want = (nrows + RW * warps - 1) / (RW * warps);
+    const int grid =
+        static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(L.sms) * per_sm)));
+    k_spmm_rows<VT, LPR, C, PLAIN><<<grid, warps * 32, epi != 0 ? smem_of(warps) : 0, L.st>>>(
+        ptr, ind, vals, static_cast<uint32_t>(nrows), X, sx, shift, Y, Z, zc, zs, epi, partials);
+    SLQ_LAUNCH_CK();
+    ++L.launches;
+    *grid_out = grid;
+    return SLQ_OK;
 }
 
-// persistent grid of the CSR kernel: as many blocks as are resident on the
-// SMs at once (a partial second wave would leave SMs idle at the end)
+// CSR product.  16-byte pieces (k_spmm_rows) from 32 probes on; the Krylov
+// driver's blocks are always aligned for them, a caller's (slq_operator_dot)
+// of 32 or 64 probes need not be.
 template <typename VT>
-int spmm_grid(const Launcher& L, int64_t nrows, int b)
-{
-    int per_sm = 4;
-    switch (b)
-    {
-        case 64: per_sm = spmm_blocks_per_sm<VT, 2, 1>(b); break;
-        case 128: per_sm = spmm_blocks_per_sm<VT, 4, 1>(b); break;
-        case 256: per_sm = spmm_blocks_per_sm<VT, 8, 1>(b); break;
-        case 512: per_sm = spmm_blocks_per_sm<VT, 16, 1>(b); break;
-        case 1024: per_sm = spmm_blocks_per_sm<VT, 32, 1>(b); break;
-        default: break;
-    }
-    const int64_t g = (nrows + 7) / 8;
-    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(g, int64_t(L.sms) * per_sm)));
-}
-
-template <typename VT>
-slq_status spmm(Launcher& L, int grid, const int32_t* ptr, const int32_t* ind, const VT* vals,
+slq_status spmm(Launcher& L, const int32_t* ptr, const int32_t* ind, const VT* vals,
                 int64_t nrows, int b, const VT* X, const double* sx, double shift, VT* Y,
                 const VT* Z, const double* zc, const double* zs, int epi, double* partials,
-                int64_t nnz, int64_t xrows)
+                int64_t nnz, int64_t xrows, int* grid_out)
 {
-#define SLQ_SPMM_CASE(BB, LV, KS)                                                         \
-    case BB:                                                                              \
-        return spmm_inst<VT, LV, KS>(L, grid, ptr, ind, vals, nrows, b, X, sx, shift, Y,  \
-                                     Z, zc, zs, epi, partials, nnz, xrows);
-    switch (b)
-    {
-        SLQ_SPMM_CASE(1, 1, 32)
-        SLQ_SPMM_CASE(2, 1, 16)
-        SLQ_SPMM_CASE(4, 1, 8)
-        SLQ_SPMM_CASE(8, 1, 4)
-        SLQ_SPMM_CASE(16, 1, 2)
-        SLQ_SPMM_CASE(32, 1, 1)
-        SLQ_SPMM_CASE(64, 2, 1)
-        SLQ_SPMM_CASE(128, 4, 1)
-        SLQ_SPMM_CASE(256, 8, 1)
-        SLQ_SPMM_CASE(512, 16, 1)
-        SLQ_SPMM_CASE(1024, 32, 1)
-        default:
-            return fail(SLQ_ERR_BAD_ARG, "block width must be a power of two <= 1024");
+    const bool aligned = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y) |
+                           reinterpret_cast<uintptr_t>(Z)) & 15) == 0;
+#define SLQ_SPMM_CASE(BB, LV, KS)                                                            \
+    if (b == BB)                                                                             \
+        return spmm_inst<VT, LV, KS>(L, ptr, ind, vals, nrows, b, X, sx, shift, Y, Z, zc, zs, \
+                                     epi, partials, nnz, xrows, grid_out);
+#define SLQ_ROWS_CASE(BB)                                                                        \
+    if (b == BB)                                                                                 \
+    {                                                                                            \
+        constexpr int lpr = BB / V < 32 ? BB / V : 32;                                           \
+        if (shift == 0.0 && !Z)                                                                  \
+            return spmm_rows_inst<VT, lpr, BB / V / lpr, true>(L, ptr, ind, vals, nrows, X, sx,  \
+                                                               shift, Y, Z, zc, zs, epi,         \
+                                                               partials, nnz, xrows, grid_out);  \
+        return spmm_rows_inst<VT, lpr, BB / V / lpr, false>(L, ptr, ind, vals, nrows, X, sx,     \
+                                                            shift, Y, Z, zc, zs, epi, partials,  \
+                                                            nnz, xrows, grid_out);               \
     }
+    constexpr int V = 16 / static_cast<int>(sizeof(VT));
+    SLQ_SPMM_CASE(1, 1, 32)
+    SLQ_SPMM_CASE(2, 1, 16)
+    SLQ_SPMM_CASE(4, 1, 8)
+    SLQ_SPMM_CASE(8, 1, 4)
+    SLQ_SPMM_CASE(16, 1, 2)
+    if (!aligned)
+    {
+        SLQ_SPMM_CASE(32, 1, 1)
+        if constexpr (sizeof(VT) == 4) { SLQ_SPMM_CASE(64, 2, 1) }
+    }
+    SLQ_ROWS_CASE(32)
+    SLQ_ROWS_CASE(64)
+    SLQ_ROWS_CASE(128)
+    SLQ_ROWS_CASE(256)
+    SLQ_ROWS_CASE(512)
+    if constexpr (sizeof(VT) == 4) { SLQ_ROWS_CASE(1024) }
+    return fail(SLQ_ERR_BAD_ARG, "block width must be a power of two <= 1024");
+#undef SLQ_ROWS_CASE
 #undef SLQ_SPMM_CASE
 }
 
@@ -1762,10 +1789,8 @@ slq_status spmm_cand(Launcher& L, const slq_op* op, int transpose, const SpmmCan
     const int32_t* ptr = transpose ? op->t_ptr : op->a_ptr;
     const int32_t* ind = transpose ? op->t_ind : op->a_ind;
     const VT* val = static_cast<const VT*>(transpose ? op->t_data : op->a_data);
-    const int grid = spmm_grid<VT>(L, rows, b);
-    *grid_out = grid;
-    return spmm<VT>(L, grid, ptr, ind, val, rows, b, X, sx, shift, Y, Z, zc, zs, epi, partials,
-                    op->nnz, xrows);
+    return spmm<VT>(L, ptr, ind, val, rows, b, X, sx, shift, Y, Z, zc, zs, epi, partials, op->nnz,
+                    xrows, grid_out);
 }
 
 int log2_width(int b)

@@ -145,14 +145,16 @@ __device__ __forceinline__ int ring_slot(int vec, int bs)
 // ---------------------------------------------------------------------------
 // CSR SpMM: Y = sx * (A X) [+ shift * sx * X] [- zc * zs * Z]
 //
-// One warp per matrix row; the row's b probe columns are split over the
-// lanes: P = b / LV lanes, each owning LV consecutive probes, and KS = 32/P
-// lane slices that walk alternate nonzeros of the row (KS > 1 only for
-// b < 32).  Column indices and values are read coalesced 32 at a time and
-// broadcast by shuffle; each nonzero then costs one contiguous LV-wide
-// gather per lane (the whole warp reads b contiguous values of X).  The
-// epilogue applies the per-probe scale and the Krylov recurrence's axpy and
-// accumulates the FP64 partial of alpha (Lanczos) or of the squared norm.
+// One warp per matrix row, for b <= 16 and for wider blocks whose buffers
+// are not 16-byte aligned (k_spmm_rows serves the rest); the row's b probe
+// columns are split over the lanes: P = b / LV lanes, each owning LV
+// consecutive probes, and KS = 32/P lane slices that walk alternate nonzeros
+// of the row (KS > 1 only for b < 32).  Column indices and values are read
+// coalesced 32 at a time and broadcast by shuffle; each nonzero then costs
+// one contiguous LV-wide gather per lane (the whole warp reads b contiguous
+// values of X).  The epilogue applies the per-probe scale and the Krylov
+// recurrence's axpy and accumulates the FP64 partial of alpha (Lanczos) or of
+// the squared norm.
 //
 // epi: 0 store only, 1 alpha partial <sx X[r], Y[r]>, 2 norm partial
 // |Y[r]|^2, 3 alpha partial <zs Z[r], Y[r]> (normal-equations Lanczos, where
@@ -163,7 +165,7 @@ __device__ __forceinline__ int ring_slot(int vec, int bs)
 // more warps keep more row gathers in flight (short rows issue few per warp)
 template <typename VT, int LV>
 struct SpmmOcc {
-    static constexpr int MINB = (sizeof(VT) != 4) ? 1 : (LV <= 4) ? 4 : (LV == 8 ? 3 : 1);
+    static constexpr int MINB = (sizeof(VT) != 4) ? 1 : 4;
 };
 
 template <typename VT, int LV, int KS>
@@ -291,6 +293,261 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
         double s = 0.0;
         for (int w = 0; w < nwarps; ++w) s += smem_spmm[w * b + p];
         partials[static_cast<int64_t>(blockIdx.x) * b + p] = s;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// CSR SpMM for blocks of 32 probes and more: the product and epilogue of
+// k_spmm, the same row sums in the same order.
+//
+// With rows of a few entries the product moves b-wide rows and little else;
+// what bounds it is the number of rows in flight and the work around them, not
+// the FMAs.  So
+// * a lane owns 16-byte pieces that are contiguous across the lanes of a row
+//   (piece c of lane l at probe (c LPR + l) VEC): one line per eight lanes,
+//   where LV consecutive probes per lane touched every line of a row twice;
+// * the scales stay in registers (read per row, they took more L1 cycles than
+//   the gathers);
+// * every lane reads a row's columns and values itself (one address per row:
+//   a broadcast) instead of 32 at a time with two shuffles per entry, U
+//   entries are gathered at once, and the next row's bounds load a row ahead;
+// * the FP32 epilogue keeps off the FP64 conversion unit (16 values per clock
+//   and SM, four conversions per element before, one now): see y_scaled and
+//   f64_of_basis.
+// LPR = min(32, b / VEC) lanes serve a row, 32 / LPR rows share a warp, C =
+// b / (VEC LPR) pieces per lane.
+// Measured (the 8-wide-lane k_spmm before, this kernel now), us per product:
+// 524,175 rows of 5 entries, b = 256, FP32: 575 -> 297 (X and Y alone: 165 at
+// the copy rate); 89,999 rows of 5, b = 128, FP64: 102 -> 56; 16,384 rows of
+// 2, b = 256, FP64, both directions: 58 -> 33; a 524,288 x 131,072 matrix
+// with 16 random entries per column, b = 128, FP32, mean of A and A^T:
+// 216 -> 172.
+// ---------------------------------------------------------------------------
+
+// x * s rounded to FP32, for s given as the FP32 pair sh + sl: the FP32
+// product and its exact remainder, which is the double product rounded to
+// FP32 up to ties (relative error before the rounding 2^-48).
+__device__ __forceinline__ float y_scaled(float x, float sh, float sl)
+{
+    const float p = x * sh;
+    return p + fmaf(x, sl, fmaf(x, sh, -p));
+}
+
+// 2^-896 x as a double, from the bits of x: exact for every finite x, zeros
+// and subnormals included (the FP32 exponent is read with the FP64 bias).  An
+// infinity or NaN becomes a finite value: only for a Krylov basis vector,
+// whose non-finite entries have already made the norm it was divided by
+// non-finite.
+__device__ __forceinline__ double f64_of_basis(float x)
+{
+    const int b = __float_as_int(x);
+    return __hiloint2double((b >> 3) & 0x8fffffff, b << 29);
+}
+constexpr double TWO_896 = 0x1p896;
+
+template <typename VT, int C>
+struct SpmmRowsShape {
+    // entries gathered at once and resident 256-thread blocks per SM: swept
+    // at the sizes above (FP32 C = 2: 5 entries at 3 blocks, 8 at 2 and 4 at 4
+    // were 10 to 40 % slower; C = 1: 8 at 4 best)
+    static constexpr int U = C == 1 ? 8 : C == 2 ? 5 : C == 4 ? 3 : 2;
+    static constexpr int MINB = C == 1 ? 4 : C == 2 ? 3 : C == 4 ? 2 : 1;
+};
+
+// PLAIN: Y = sx * (A X) alone (no shift, no Z; epi 0, 1 or 2)
+template <typename VT, int LPR, int C, bool PLAIN>
+__global__ void __launch_bounds__(256, SpmmRowsShape<VT, C>::MINB)
+k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+            const VT* __restrict__ vals, uint32_t nrows, const VT* __restrict__ X,
+            const double* __restrict__ sx, double shift, VT* __restrict__ Y,
+            const VT* __restrict__ Z, const double* __restrict__ zc,
+            const double* __restrict__ zs, int epi, double* __restrict__ partials)
+{
+    constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+    constexpr int RW = 32 / LPR;          // rows per warp
+    constexpr int b = LPR * VEC * C;
+    constexpr int U = SpmmRowsShape<VT, C>::U;
+    constexpr int LV = C * VEC;
+    constexpr bool F32 = sizeof(VT) == 4;
+    extern __shared__ double smem_rows[];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int nwarps = blockDim.x >> 5;
+    const int rl = lane % LPR;            // lane within the row
+    const int rs = lane / LPR;            // row within the warp
+    auto probe = [&](int v) { return ((v / VEC) * LPR + rl) * VEC + v % VEC; };
+    // s_p; FP32 plain products: s_p as an FP32 pair in the same registers
+    double sxr[LV], part[LV];
+#pragma unroll
+    for (int v = 0; v < LV; ++v)
+    {
+        const double s = sx ? sx[probe(v)] : 1.0;
+        part[v] = 0.0;
+        if constexpr (F32 && PLAIN)
+        {
+            const float sh = static_cast<float>(s);
+            const float sl = isinf(sh) ? 0.0f : static_cast<float>(s - static_cast<double>(sh));
+            sxr[v] = __hiloint2double(__float_as_int(sh), __float_as_int(sl));
+        }
+        else
+            sxr[v] = s;
+    }
+    auto scale_h = [&](int v) { return __int_as_float(__double2hiint(sxr[v])); };
+    auto scale_l = [&](int v) { return __int_as_float(__double2loint(sxr[v])); };
+
+    const VT* Xl = X + rl * VEC;
+    // 32-bit rows (nrows < 2^31, and a stride more still fits)
+    const uint32_t stride = gridDim.x * nwarps * RW;
+    uint32_t row = (blockIdx.x * nwarps + warp) * RW + rs;
+    int n0 = 0, n1 = 0;
+    if (row < nrows)
+    {
+        n0 = __ldg(indptr + row);
+        n1 = __ldg(indptr + row + 1);
+    }
+    // row - rs < nrows keeps the warp's loop uniform
+    for (; row - rs < nrows; row += stride)
+    {
+        const bool live = row < nrows;
+        const int k1 = n1;
+        int k = n0;
+        n0 = n1 = 0;
+        if (row + stride < nrows)
+        {
+            n0 = __ldg(indptr + row + stride);
+            n1 = __ldg(indptr + row + stride + 1);
+        }
+        VT acc[LV];
+#pragma unroll
+        for (int v = 0; v < LV; ++v) acc[v] = VT(0);
+        for (;; k += U)
+        {
+            const int cnt = k1 - k;
+            if constexpr (RW > 1)
+            {
+                if (!__any_sync(FULL_MASK, cnt > 0)) break;
+            }
+            else
+            {
+                if (cnt <= 0) break;
+            }
+            int cc[U];
+            VT aa[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                cc[u] = 0;
+                aa[u] = VT(0);
+                if (u < cnt)
+                {
+                    cc[u] = __ldg(indices + k + u);
+                    aa[u] = __ldg(vals + k + u);
+                }
+            }
+            VT x[U][LV];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < C; ++q)
+                {
+                    VT piece[VEC];
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) piece[v] = VT(0);
+                    if (u < cnt)
+                        ldg_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) x[u][q * VEC + v] = piece[v];
+                }
+            // entries past the row's end add 0 * 0
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < LV; ++v) acc[v] += aa[u] * x[u][v];
+        }
+        if (!live) continue;
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+        {
+            const size_t o = static_cast<size_t>(row) * b + (q * LPR + rl) * VEC;
+            VT xr[VEC], yr[VEC];
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) xr[v] = VT(0);
+            if ((!PLAIN && shift != 0.0) || epi == 1) ldg_n<VT, VEC>(X + o, xr);
+            if constexpr (PLAIN)
+            {
+#pragma unroll
+                for (int v = 0; v < VEC; ++v)
+                {
+                    const int w = q * VEC + v;
+                    // without a scale the product is stored as it is (an
+                    // infinity would not pass y_scaled)
+                    if constexpr (F32)
+                        yr[v] = sx ? y_scaled(acc[w], scale_h(w), scale_l(w)) : acc[w];
+                    else
+                        yr[v] = acc[w] * sxr[w];
+                }
+                if (epi == 1)
+                {
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v)
+                    {
+                        if constexpr (F32)
+                            part[q * VEC + v] +=
+                                f64_of_basis(xr[v]) * (static_cast<double>(yr[v]) * TWO_896);
+                        else
+                            part[q * VEC + v] += xr[v] * yr[v];
+                    }
+                }
+                else if (epi == 2)
+                {
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v)
+                        part[q * VEC + v] +=
+                            static_cast<double>(yr[v]) * static_cast<double>(yr[v]);
+                }
+            }
+            else
+            {
+                VT zr[VEC];
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) zr[v] = VT(0);
+                const int p0 = (q * LPR + rl) * VEC;
+                if (Z) ldg_n<VT, VEC>(Z + o, zr);
+#pragma unroll
+                for (int v = 0; v < VEC; ++v)
+                {
+                    const int w = q * VEC + v;
+                    const double s = sxr[w];
+                    double y = static_cast<double>(acc[w]) * s;
+                    if (shift != 0.0) y += shift * (s * static_cast<double>(xr[v]));
+                    if (Z)
+                        y -= (__ldg(zc + p0 + v) * __ldg(zs + p0 + v)) * static_cast<double>(zr[v]);
+                    yr[v] = static_cast<VT>(y);
+                    const double ys = static_cast<double>(yr[v]);
+                    if (epi == 1)
+                        part[w] += static_cast<double>(xr[v]) * ys;
+                    else if (epi == 2)
+                        part[w] += ys * ys;
+                    else if (epi == 3)
+                        part[w] += static_cast<double>(zr[v]) * ys;
+                }
+            }
+            store_n<VT, VEC>(Y + o, yr);
+        }
+    }
+
+    if (epi == 0) return;
+    // CTA reduction over warps and the rows of a warp, fixed order; then the
+    // per-probe factor of the terms (s_p, 1 or zs_p)
+#pragma unroll
+    for (int v = 0; v < LV; ++v) smem_rows[(warp * RW + rs) * b + probe(v)] = part[v];
+    __syncthreads();
+    for (int p = threadIdx.x; p < b; p += blockDim.x)
+    {
+        double s = 0.0;
+        for (int w = 0; w < nwarps * RW; ++w) s += smem_rows[w * b + p];
+        const double f = epi == 1 ? (sx ? sx[p] : 1.0) : epi == 3 ? zs[p] : 1.0;
+        partials[static_cast<int64_t>(blockIdx.x) * b + p] = f * s;
     }
 }
 
