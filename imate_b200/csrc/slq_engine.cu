@@ -1178,17 +1178,22 @@ slq_status spmm_rows_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, c
     return SLQ_OK;
 }
 
+inline bool aligned16(const void* a, const void* b, const void* c)
+{
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
+             reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+
 // CSR product.  16-byte pieces (k_spmm_rows) from 32 probes on; the Krylov
 // driver's blocks are always aligned for them, a caller's (slq_operator_dot)
-// of 32 or 64 probes need not be.
+// need not be.
 template <typename VT>
 slq_status spmm(Launcher& L, const int32_t* ptr, const int32_t* ind, const VT* vals,
                 int64_t nrows, int b, const VT* X, const double* sx, double shift, VT* Y,
                 const VT* Z, const double* zc, const double* zs, int epi, double* partials,
                 int64_t nnz, int64_t xrows, int* grid_out)
 {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y) |
-                           reinterpret_cast<uintptr_t>(Z)) & 15) == 0;
+    const bool aligned = aligned16(X, Y, Z);
 #define SLQ_SPMM_CASE(BB, LV, KS)                                                            \
     if (b == BB)                                                                             \
         return spmm_inst<VT, LV, KS>(L, ptr, ind, vals, nrows, b, X, sx, shift, Y, Z, zc, zs, \
@@ -1213,8 +1218,14 @@ slq_status spmm(Launcher& L, const int32_t* ptr, const int32_t* ind, const VT* v
     SLQ_SPMM_CASE(16, 1, 2)
     if (!aligned)
     {
-        SLQ_SPMM_CASE(32, 1, 1)
-        if constexpr (sizeof(VT) == 4) { SLQ_SPMM_CASE(64, 2, 1) }
+        // 32 columns at a time; only slq_operator_dot comes here (no
+        // partial sums)
+        if (epi != 0) return fail(SLQ_ERR_BAD_ARG, "SpMM: the probe block is not aligned");
+        for (int p = 0; p < b; p += 32)
+            SLQ_TRY(spmm_inst<VT, 1, 1>(L, ptr, ind, vals, nrows, b, X + p, sx ? sx + p : nullptr,
+                                        shift, Y + p, Z ? Z + p : nullptr, zc ? zc + p : nullptr,
+                                        zs ? zs + p : nullptr, 0, nullptr, nnz, xrows, grid_out));
+        return SLQ_OK;
     }
     SLQ_ROWS_CASE(32)
     SLQ_ROWS_CASE(64)
@@ -1498,29 +1509,68 @@ slq_status spmm_rgt_inst(Launcher& L, const CUtensorMap* xmap, const int32_t* gp
     return SLQ_OK;
 }
 
-// Operator product on a block: row-group SpMM where the operator has the
-// format and the width suits it (32 <= b <= 256; FP64 b <= 128), else CSR.
-// *grid_out receives the number of partial rows the launch writes.
-template <typename VT, int LV, int G, int NS>
+template <typename VT, int LPR, int RPW, bool PLAIN>
 slq_status spmm_rg_inst(Launcher& L, const int32_t* gptr, const int32_t* gcol, const VT* gval,
-                        int64_t nrows, int b, const VT* X, const double* sx, double shift, VT* Y,
-                        const VT* Z, const double* zc, const double* zs, int epi,
+                        int64_t nrows, int G, int b, const VT* X, const double* sx, double shift,
+                        VT* Y, const VT* Z, const double* zc, const double* zs, int epi,
                         double* partials, int64_t nnz, int64_t xrows, int* grid_out)
 {
-    const double s = sizeof(VT);
-    const double bytes = nnz * (s + 4.0) + (nrows + 1) * 4.0 + double(xrows) * b * s +
-                         double(nrows) * b * s * (Z ? 2.0 : 1.0);
-    ProfScope prof(SLQ_K_SPMM, bytes, L.st);
+    constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+    constexpr int RW = 32 / LPR;
+    ProfScope prof(SLQ_K_SPMM, spmm_bytes<VT>(nnz, nrows, xrows, b, Z != nullptr), L.st);
     const int64_t ng = (nrows + G - 1) / G;
-    constexpr int GPC = 8 / NS;
-    const int grid = static_cast<int>(
-        std::max<int64_t>(1, std::min<int64_t>((ng + GPC - 1) / GPC, int64_t(L.sms) * 4)));
-    k_spmm_rg<VT, LV, G, NS><<<grid, 256, 0, L.st>>>(gptr, gcol, gval, nrows, ng, b, X, sx, shift, Y,
-                                                 Z, zc, zs, epi, partials);
+    const int slices = b / (VEC * LPR);
+    const int64_t items = ng * (G / RPW);
+    static std::atomic<int> resident{0};
+    int per_sm = resident.load();
+    if (per_sm == 0)
+    {
+        int v = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_spmm_rg<VT, LPR, RPW, PLAIN>, 256,
+                                                          8 * 1024) != cudaSuccess ||
+            v < 1)
+            v = 1;
+        per_sm = std::min(v, 4);
+        resident.store(per_sm);
+    }
+    // smaller blocks where there are fewer items than the SMs have warps
+    int warps = 8;
+    while (warps > slices && warps > 1 && items * slices <= int64_t(L.sms) * RW * warps / 2)
+        warps >>= 1;
+    const int64_t per_cta = int64_t(warps) / slices * RW;
+    const size_t smem = epi != 0 ? static_cast<size_t>(per_cta) * b * sizeof(double) : 0;
+    const int grid = static_cast<int>(std::max<int64_t>(
+        1, std::min<int64_t>((items + per_cta - 1) / per_cta, int64_t(L.sms) * per_sm)));
+    k_spmm_rg<VT, LPR, RPW, PLAIN><<<grid, warps * 32, smem, L.st>>>(
+        gptr, gcol, gval, static_cast<uint32_t>(nrows), static_cast<uint32_t>(ng), G, b, X, sx,
+        shift, Y, Z, zc, zs, epi, partials);
     SLQ_LAUNCH_CK();
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
+}
+
+template <typename VT, int LPR>
+slq_status spmm_rg(Launcher& L, int rpw, const int32_t* gptr, const int32_t* gcol, const VT* gval,
+                   int64_t nrows, int G, int b, const VT* X, const double* sx, double shift, VT* Y,
+                   const VT* Z, const double* zc, const double* zs, int epi, double* partials,
+                   int64_t nnz, int64_t xrows, int* grid_out)
+{
+#define SLQ_RG_CASE(RPW)                                                                        \
+    if (rpw == RPW)                                                                             \
+    {                                                                                           \
+        if (shift == 0.0 && !Z)                                                                 \
+            return spmm_rg_inst<VT, LPR, RPW, true>(L, gptr, gcol, gval, nrows, G, b, X, sx,    \
+                                                    shift, Y, Z, zc, zs, epi, partials, nnz,    \
+                                                    xrows, grid_out);                           \
+        return spmm_rg_inst<VT, LPR, RPW, false>(L, gptr, gcol, gval, nrows, G, b, X, sx,       \
+                                                 shift, Y, Z, zc, zs, epi, partials, nnz,       \
+                                                 xrows, grid_out);                              \
+    }
+    SLQ_RG_CASE(4)
+    SLQ_RG_CASE(8)
+#undef SLQ_RG_CASE
+    return fail(SLQ_ERR_BAD_ARG, "row-group SpMM: unsupported tile");
 }
 
 // Tensor-core row-group SpMM (k_spmm_tc): 16-row groups, b = 128 NS, two
@@ -1665,6 +1715,7 @@ enum { CAND_CSR = 0, CAND_RG = 1, CAND_TMA = 2, CAND_TC = 3, CAND_BLK = 4 };
 
 struct SpmmCand {
     int kind, g, lv, ns;
+    int rpw = 0;  // CAND_RG: rows of the group per warp
 };
 
 template <typename VT>
@@ -1677,16 +1728,13 @@ int spmm_candidates(const slq_op* op, int transpose, int b, SpmmCand* out)
     const int32_t* gptr = transpose ? op->t_gptr : op->a_gptr;
     const int G = op->group_rows;
     if (!G || !gptr) return n;
-    // FP64 row groups: b <= 64, LV <= 2, G <= 8 (shared-memory staging);
-    // 16-row groups keep LV <= 2 (16 x LV accumulators per lane)
-    const int bmax = (sizeof(VT) == 8) ? 64 : 256;
-    const int lvmax = (sizeof(VT) == 8 || G == 16) ? 2 : 4;
-    if (b >= 32 && b <= bmax && (sizeof(VT) == 4 || G <= 8))
-        for (int lv = 1; lv <= lvmax; lv *= 2)
-        {
-            const int ns = b / (32 * lv);
-            if (ns >= 1 && ns <= 8 && 32 * lv * ns == b) out[n++] = {CAND_RG, G, lv, ns};
-        }
+    // row groups from 32 probes on (FP64: groups of at most 8 rows); a warp
+    // takes 4 or 8 of the group's rows and the probes of its lanes' 16-byte
+    // pieces
+    const int vec = 16 / static_cast<int>(sizeof(VT));
+    if (b >= 32 && (sizeof(VT) == 4 || G <= 8))
+        for (int rpw = 4; rpw <= std::min(G, 8); rpw *= 2)
+            out[n++] = {CAND_RG, G, vec, std::max(1, G / rpw * b / (32 * vec)), rpw};
     if (sizeof(VT) == 4 && (G == 8 || G == 16) && (b == 128 || b == 256))
         out[n++] = {CAND_TMA, G, 4, b / 128};
     if (sizeof(VT) == 4 && G == 16 && (b == 128 || b == 256))
@@ -1752,39 +1800,17 @@ slq_status spmm_cand(Launcher& L, const slq_op* op, int transpose, const SpmmCan
     if (c.kind == CAND_RG)
     {
         const VT* gval = static_cast<const VT*>(transpose ? op->t_gval : op->a_gval);
-#define SLQ_RG_CASE(GG, LVV, NSS)                                                            \
-    if (c.g == GG && c.lv == LVV && c.ns == NSS)                                           \
-        return spmm_rg_inst<VT, LVV, GG, NSS>(L, gptr, gcol, gval, rows, b, X, sx, shift, Y, \
-                                              Z, zc, zs, epi, partials, op->nnz, xrows,     \
-                                              grid_out);
-#define SLQ_RG_ALL(GG)         \
-    SLQ_RG_CASE(GG, 1, 1)      \
-    SLQ_RG_CASE(GG, 1, 2)      \
-    SLQ_RG_CASE(GG, 2, 1)      \
-    if constexpr (sizeof(VT) == 4) \
-    {                          \
-        SLQ_RG_CASE(GG, 1, 4)  \
-        SLQ_RG_CASE(GG, 2, 2)  \
-        SLQ_RG_CASE(GG, 4, 1)  \
-        SLQ_RG_CASE(GG, 1, 8)  \
-        SLQ_RG_CASE(GG, 2, 4)  \
-        SLQ_RG_CASE(GG, 4, 2)  \
-    }
-        SLQ_RG_ALL(8)
-        SLQ_RG_ALL(4)
-        if constexpr (sizeof(VT) == 4)
-        {
-            SLQ_RG_CASE(16, 1, 1)
-            SLQ_RG_CASE(16, 1, 2)
-            SLQ_RG_CASE(16, 2, 1)
-            SLQ_RG_CASE(16, 1, 4)
-            SLQ_RG_CASE(16, 2, 2)
-            SLQ_RG_CASE(16, 1, 8)
-            SLQ_RG_CASE(16, 2, 4)
-        }
-#undef SLQ_RG_ALL
-#undef SLQ_RG_CASE
-        return fail(SLQ_ERR_BAD_ARG, "row-group SpMM: unsupported tile");
+        constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+        if (b >= 32 * VEC)
+            return spmm_rg<VT, 32>(L, c.rpw, gptr, gcol, gval, rows, c.g, b, X, sx, shift, Y, Z, zc,
+                                   zs, epi, partials, op->nnz, xrows, grid_out);
+        if (b == 16 * VEC)
+            return spmm_rg<VT, 16>(L, c.rpw, gptr, gcol, gval, rows, c.g, b, X, sx, shift, Y, Z, zc,
+                                   zs, epi, partials, op->nnz, xrows, grid_out);
+        if constexpr (VEC == 4)
+            return spmm_rg<VT, 8>(L, c.rpw, gptr, gcol, gval, rows, c.g, b, X, sx, shift, Y, Z, zc,
+                                  zs, epi, partials, op->nnz, xrows, grid_out);
+        return fail(SLQ_ERR_BAD_ARG, "row-group SpMM: unsupported width");
     }
     const int32_t* ptr = transpose ? op->t_ptr : op->a_ptr;
     const int32_t* ind = transpose ? op->t_ind : op->a_ind;
@@ -1798,6 +1824,41 @@ int log2_width(int b)
     int lg = 0;
     while ((1 << lg) < b) ++lg;
     return lg;
+}
+
+// The product of an operator without a block format and without a tuned
+// choice: CSR or row groups (rpw rows of a group per warp) or their TMA form,
+// by rows, group width and block width.  Measured on correlation matrices
+// with L2 flushed between products, as the passes over the basis leave it, us
+// (CSR / row groups; TMA after a slash of its own):
+//   FP32, 8-row groups   n 8,000 b 64: 14 / 47, b 256: 29 / 53; n 16,400 b 64:
+//                        27 / 27, b 128: 35 / 31; n 30,011 b 256: 64 / 62; n
+//                        65,537 b 64: 74 / 70, b 128: 113 / 94 / 90, b 256:
+//                        181 / 154 / 164; n 150,000 b 128: 135 / 127 / 137
+//   FP32, 16-row groups  n 32,768 b 64: 61 / 104, b 256: 152 / 197 / 198; n
+//                        50,000 b 256: 275 / 294 / 256; n 100,003 b 64: 152 /
+//                        172, b 128: 246 / 244 / 219, b 256: 398 / 423 / 342;
+//                        n 262,144 b 32: 459 / 401, b 64: 793 / 557, b 128:
+//                        1,214 / 895 / 682
+//   FP64, 8-row groups   n 17,000 b 64: 35 / 37; n 40,009 b 64: 80 / 98; n
+//                        100,000 b 32: 88 / 107, b 64: 133 / 146
+// Small matrices have too few groups to hide a gather's latency, and FP64
+// groups lose by their padding at every size.
+struct SpmmRule {
+    int kind, rpw;
+};
+
+template <typename VT>
+SpmmRule spmm_rule(int64_t rows, int G, int b)
+{
+    const SpmmRule csr{CAND_CSR, 0}, groups{CAND_RG, std::min(G, 8)};
+    if (sizeof(VT) == 8 || !G || rows < 16384 || b < 32 || b > 256) return csr;
+    if (G == 16)
+    {
+        if (b >= 128) return rows >= (b == 128 ? 65536 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
+        return rows >= 200000 ? groups : csr;
+    }
+    return (b >= 128 || rows >= 65536) ? groups : csr;
 }
 
 // Operator product on a block.  An autotuned choice (slq_operator_tune /
@@ -1827,33 +1888,25 @@ slq_status op_spmm(Launcher& L, const slq_op* op, int transpose, int b, const VT
     auto usable = [&](const SpmmCand& c) {
         if (c.kind == CAND_TMA || c.kind == CAND_TC) return have_row;
         if (c.kind == CAND_BLK) return have_blk;
+        if (c.kind == CAND_RG) return aligned16(X, Y, Z);
         return true;
     };
     if (ti >= 0 && ti < nc && usable(cands[ti]))
         return spmm_cand<VT>(L, op, transpose, cands[ti], b, X, sx, shift, Y, Z, zc, zs, epi,
                              partials, grid_out, maps, error);
-    // built-in choice: the tensor-core block kernel, TMA, then the row-group
-    // tile with the widest LV, then CSR
+    // built-in choice: the tensor-core block kernel where the operator has the
+    // format, else by spmm_rule, else CSR
+    const int64_t rows = transpose ? op->ncols : op->nrows;
     int pick = 0;
     for (int i = 0; i < nc; ++i)
+        if (cands[i].kind == CAND_BLK && have_blk) pick = i;
+    if (cands[pick].kind != CAND_BLK)
     {
-        if (cands[i].kind == CAND_BLK && have_blk)
-        {
-            pick = i;
-            break;
-        }
-    }
-    for (int i = 0; i < nc && cands[pick].kind != CAND_BLK; ++i)
-    {
-        if (cands[i].kind == CAND_TC || cands[i].kind == CAND_BLK) continue;  // tuner / above
-        if (cands[i].kind == CAND_TMA && !have_row) continue;
-        if (cands[i].kind == CAND_TMA)
-        {
-            pick = i;
-            break;
-        }
-        if (cands[i].kind == CAND_RG && (cands[pick].kind != CAND_RG || cands[i].lv > cands[pick].lv))
-            pick = i;
+        const SpmmRule want = spmm_rule<VT>(rows, op->group_rows, b);
+        for (int i = 0; i < nc; ++i)
+            if (usable(cands[i]) && cands[i].kind == want.kind &&
+                (want.kind != CAND_RG || cands[i].rpw == want.rpw))
+                pick = i;
     }
     return spmm_cand<VT>(L, op, transpose, cands[pick], b, X, sx, shift, Y, Z, zc, zs, epi,
                          partials, grid_out, maps, error);

@@ -145,11 +145,11 @@ __device__ __forceinline__ int ring_slot(int vec, int bs)
 // ---------------------------------------------------------------------------
 // CSR SpMM: Y = sx * (A X) [+ shift * sx * X] [- zc * zs * Z]
 //
-// One warp per matrix row, for b <= 16 and for wider blocks whose buffers
-// are not 16-byte aligned (k_spmm_rows serves the rest); the row's b probe
-// columns are split over the lanes: P = b / LV lanes, each owning LV
-// consecutive probes, and KS = 32/P lane slices that walk alternate nonzeros
-// of the row (KS > 1 only for b < 32).  Column indices and values are read
+// One warp per matrix row, for b <= 16 and, 32 columns at a time, for wider
+// blocks whose buffers are not 16-byte aligned (k_spmm_rows serves the rest);
+// the row's probe columns are split over the lanes: P = 32 / KS lanes, each
+// owning LV = 1 probe, and KS lane slices that walk alternate nonzeros of the
+// row (KS > 1 only for b < 32).  Column indices and values are read
 // coalesced 32 at a time and broadcast by shuffle; each nonzero then costs
 // one contiguous LV-wide gather per lane (the whole warp reads b contiguous
 // values of X).  The epilogue applies the per-probe scale and the Krylov
@@ -324,6 +324,16 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
 // 216 -> 172.
 // ---------------------------------------------------------------------------
 
+// L2 prefetch of [p, p + bytes) by n lanes (lane 0 .. n - 1), a 128-byte line
+// each: the matrix streams past once per product, and between products the
+// Krylov basis has pushed it out of L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes, int lane, int n)
+{
+    const char* q = static_cast<const char*>(p);
+    for (int64_t o = static_cast<int64_t>(lane) * 128; o < bytes; o += n * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+}
+
 // x * s rounded to FP32, for s given as the FP32 pair sh + sl: the FP32
 // product and its exact remainder, which is the double product rounded to
 // FP32 up to ties (relative error before the rounding 2^-48).
@@ -344,6 +354,93 @@ __device__ __forceinline__ double f64_of_basis(float x)
     return __hiloint2double((b >> 3) & 0x8fffffff, b << 29);
 }
 constexpr double TWO_896 = 0x1p896;
+
+// The per-probe scales of a lane's C x VEC probes: s_p, or for FP32 products
+// without shift and Z (PLAIN) s_p as an FP32 pair in the same registers.
+template <typename VT, bool PLAIN>
+__device__ __forceinline__ double pack_scale(double s)
+{
+    if constexpr (sizeof(VT) == 4 && PLAIN)
+    {
+        const float sh = static_cast<float>(s);
+        const float sl = isinf(sh) ? 0.0f : static_cast<float>(s - static_cast<double>(sh));
+        return __hiloint2double(__float_as_int(sh), __float_as_int(sl));
+    }
+    else
+        return s;
+}
+
+// One 16-byte piece of a finished row: y = s acc [+ t s x] [- zc zs z] stored
+// at Y + o, its partial-sum term added to part (the per-probe factor s_p or
+// zs_p of the terms is applied to the sums).  p0 = the piece's first probe.
+template <typename VT, bool PLAIN, int VEC = 16 / static_cast<int>(sizeof(VT))>
+__device__ __forceinline__ void finish_piece(const VT* acc, size_t o, int p0, const double* sxr,
+                                             bool scaled, double shift, const VT* X, VT* Y,
+                                             const VT* Z, const double* zc, const double* zs,
+                                             int epi, double* part)
+{
+    constexpr bool F32 = sizeof(VT) == 4;
+    VT xr[VEC], yr[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) xr[v] = VT(0);
+    if ((!PLAIN && shift != 0.0) || epi == 1) ldg_n<VT, VEC>(X + o, xr);
+    if constexpr (PLAIN)
+    {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+        {
+            // without a scale the product is stored as it is (an infinity
+            // would not pass y_scaled)
+            if constexpr (F32)
+                yr[v] = scaled ? y_scaled(acc[v], __int_as_float(__double2hiint(sxr[v])),
+                                          __int_as_float(__double2loint(sxr[v])))
+                               : acc[v];
+            else
+                yr[v] = acc[v] * sxr[v];
+        }
+        if (epi == 1)
+        {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v)
+            {
+                if constexpr (F32)
+                    part[v] += f64_of_basis(xr[v]) * (static_cast<double>(yr[v]) * TWO_896);
+                else
+                    part[v] += xr[v] * yr[v];
+            }
+        }
+        else if (epi == 2)
+        {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v)
+                part[v] += static_cast<double>(yr[v]) * static_cast<double>(yr[v]);
+        }
+    }
+    else
+    {
+        VT zr[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) zr[v] = VT(0);
+        if (Z) ldg_n<VT, VEC>(Z + o, zr);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+        {
+            const double s = sxr[v];
+            double y = static_cast<double>(acc[v]) * s;
+            if (shift != 0.0) y += shift * (s * static_cast<double>(xr[v]));
+            if (Z) y -= (__ldg(zc + p0 + v) * __ldg(zs + p0 + v)) * static_cast<double>(zr[v]);
+            yr[v] = static_cast<VT>(y);
+            const double ys = static_cast<double>(yr[v]);
+            if (epi == 1)
+                part[v] += static_cast<double>(xr[v]) * ys;
+            else if (epi == 2)
+                part[v] += ys * ys;
+            else if (epi == 3)
+                part[v] += static_cast<double>(zr[v]) * ys;
+        }
+    }
+    store_n<VT, VEC>(Y + o, yr);
+}
 
 template <typename VT, int C>
 struct SpmmRowsShape {
@@ -368,7 +465,6 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
     constexpr int b = LPR * VEC * C;
     constexpr int U = SpmmRowsShape<VT, C>::U;
     constexpr int LV = C * VEC;
-    constexpr bool F32 = sizeof(VT) == 4;
     extern __shared__ double smem_rows[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -376,24 +472,13 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
     const int rl = lane % LPR;            // lane within the row
     const int rs = lane / LPR;            // row within the warp
     auto probe = [&](int v) { return ((v / VEC) * LPR + rl) * VEC + v % VEC; };
-    // s_p; FP32 plain products: s_p as an FP32 pair in the same registers
     double sxr[LV], part[LV];
 #pragma unroll
     for (int v = 0; v < LV; ++v)
     {
-        const double s = sx ? sx[probe(v)] : 1.0;
+        sxr[v] = pack_scale<VT, PLAIN>(sx ? sx[probe(v)] : 1.0);
         part[v] = 0.0;
-        if constexpr (F32 && PLAIN)
-        {
-            const float sh = static_cast<float>(s);
-            const float sl = isinf(sh) ? 0.0f : static_cast<float>(s - static_cast<double>(sh));
-            sxr[v] = __hiloint2double(__float_as_int(sh), __float_as_int(sl));
-        }
-        else
-            sxr[v] = s;
     }
-    auto scale_h = [&](int v) { return __int_as_float(__double2hiint(sxr[v])); };
-    auto scale_l = [&](int v) { return __int_as_float(__double2loint(sxr[v])); };
 
     const VT* Xl = X + rl * VEC;
     // 32-bit rows (nrows < 2^31, and a stride more still fits)
@@ -405,10 +490,8 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
         n0 = __ldg(indptr + row);
         n1 = __ldg(indptr + row + 1);
     }
-    // row - rs < nrows keeps the warp's loop uniform
-    for (; row - rs < nrows; row += stride)
+    for (; row < nrows; row += stride)
     {
-        const bool live = row < nrows;
         const int k1 = n1;
         int k = n0;
         n0 = n1 = 0;
@@ -420,21 +503,41 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
         VT acc[LV];
 #pragma unroll
         for (int v = 0; v < LV; ++v) acc[v] = VT(0);
-        for (;; k += U)
+        // U entries at once, without predicates while the row has them
+        for (; k + U <= k1; k += U)
         {
-            const int cnt = k1 - k;
-            if constexpr (RW > 1)
-            {
-                if (!__any_sync(FULL_MASK, cnt > 0)) break;
-            }
-            else
-            {
-                if (cnt <= 0) break;
-            }
             int cc[U];
-            VT aa[U];
+            VT aa[U], x[U][LV];
 #pragma unroll
             for (int u = 0; u < U; ++u)
+            {
+                cc[u] = __ldg(indices + k + u);
+                aa[u] = __ldg(vals + k + u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < C; ++q)
+                {
+                    VT piece[VEC];
+                    ldg_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) x[u][q * VEC + v] = piece[v];
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < LV; ++v) acc[v] += aa[u] * x[u][v];
+        }
+        if (U > 1 && k < k1)
+        {
+            // the row's last entries; places past its end add 0 * 0
+            const int cnt = k1 - k;
+            constexpr int R = U > 1 ? U - 1 : 1;
+            int cc[R];
+            VT aa[R], x[R][LV];
+#pragma unroll
+            for (int u = 0; u < R; ++u)
             {
                 cc[u] = 0;
                 aa[u] = VT(0);
@@ -444,9 +547,8 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
                     aa[u] = __ldg(vals + k + u);
                 }
             }
-            VT x[U][LV];
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int u = 0; u < R; ++u)
 #pragma unroll
                 for (int q = 0; q < C; ++q)
                 {
@@ -458,81 +560,18 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) x[u][q * VEC + v] = piece[v];
                 }
-            // entries past the row's end add 0 * 0
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int u = 0; u < R; ++u)
 #pragma unroll
                 for (int v = 0; v < LV; ++v) acc[v] += aa[u] * x[u][v];
         }
-        if (!live) continue;
 #pragma unroll
         for (int q = 0; q < C; ++q)
         {
-            const size_t o = static_cast<size_t>(row) * b + (q * LPR + rl) * VEC;
-            VT xr[VEC], yr[VEC];
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) xr[v] = VT(0);
-            if ((!PLAIN && shift != 0.0) || epi == 1) ldg_n<VT, VEC>(X + o, xr);
-            if constexpr (PLAIN)
-            {
-#pragma unroll
-                for (int v = 0; v < VEC; ++v)
-                {
-                    const int w = q * VEC + v;
-                    // without a scale the product is stored as it is (an
-                    // infinity would not pass y_scaled)
-                    if constexpr (F32)
-                        yr[v] = sx ? y_scaled(acc[w], scale_h(w), scale_l(w)) : acc[w];
-                    else
-                        yr[v] = acc[w] * sxr[w];
-                }
-                if (epi == 1)
-                {
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v)
-                    {
-                        if constexpr (F32)
-                            part[q * VEC + v] +=
-                                f64_of_basis(xr[v]) * (static_cast<double>(yr[v]) * TWO_896);
-                        else
-                            part[q * VEC + v] += xr[v] * yr[v];
-                    }
-                }
-                else if (epi == 2)
-                {
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v)
-                        part[q * VEC + v] +=
-                            static_cast<double>(yr[v]) * static_cast<double>(yr[v]);
-                }
-            }
-            else
-            {
-                VT zr[VEC];
-#pragma unroll
-                for (int v = 0; v < VEC; ++v) zr[v] = VT(0);
-                const int p0 = (q * LPR + rl) * VEC;
-                if (Z) ldg_n<VT, VEC>(Z + o, zr);
-#pragma unroll
-                for (int v = 0; v < VEC; ++v)
-                {
-                    const int w = q * VEC + v;
-                    const double s = sxr[w];
-                    double y = static_cast<double>(acc[w]) * s;
-                    if (shift != 0.0) y += shift * (s * static_cast<double>(xr[v]));
-                    if (Z)
-                        y -= (__ldg(zc + p0 + v) * __ldg(zs + p0 + v)) * static_cast<double>(zr[v]);
-                    yr[v] = static_cast<VT>(y);
-                    const double ys = static_cast<double>(yr[v]);
-                    if (epi == 1)
-                        part[w] += static_cast<double>(xr[v]) * ys;
-                    else if (epi == 2)
-                        part[w] += ys * ys;
-                    else if (epi == 3)
-                        part[w] += static_cast<double>(zr[v]) * ys;
-                }
-            }
-            store_n<VT, VEC>(Y + o, yr);
+            const int p0 = (q * LPR + rl) * VEC;
+            finish_piece<VT, PLAIN>(acc + q * VEC, static_cast<size_t>(row) * b + p0, p0,
+                                    sxr + q * VEC, sx != nullptr, shift, X, Y, Z, zc, zs, epi,
+                                    part + q * VEC);
         }
     }
 
@@ -2282,144 +2321,142 @@ __global__ void k_rg_fill(const int32_t* __restrict__ ptr, const int32_t* __rest
     }
 }
 
-// Epilogue of one output row (lanes own LV consecutive probes each).
-template <typename VT, int LV>
-__device__ __forceinline__ void spmm_row_epilogue(int64_t row, int b, int p0, const VT (&acc)[LV],
-                                                  const double (&sxr)[LV],
-                                                  const double (&zcr)[LV], double shift,
-                                                  const VT* __restrict__ X, VT* __restrict__ Y,
-                                                  const VT* __restrict__ Z,
-                                                  const double* __restrict__ zs, int epi,
-                                                  double (&part)[LV])
-{
-    const int64_t o = row * b + p0;
-    VT xr[LV], zr[LV], yr[LV];
-    if (shift != 0.0 || epi == 1) ldg_n<VT, LV>(X + o, xr);
-    if (Z) ldg_n<VT, LV>(Z + o, zr);
-#pragma unroll
-    for (int v = 0; v < LV; ++v)
-    {
-        double y = static_cast<double>(acc[v]) * sxr[v];
-        if (shift != 0.0) y += shift * (sxr[v] * static_cast<double>(xr[v]));
-        if (Z) y -= zcr[v] * static_cast<double>(zr[v]);
-        yr[v] = static_cast<VT>(y);
-        const double ys = static_cast<double>(yr[v]);
-        if (epi == 1)
-            part[v] += (sxr[v] * static_cast<double>(xr[v])) * ys;
-        else if (epi == 2)
-            part[v] += ys * ys;
-        else if (epi == 3)
-            part[v] += (zs[p0 + v] * static_cast<double>(zr[v])) * ys;
-    }
-    store_n<VT, LV>(Y + o, yr);
-}
+// One item is RPW of a group's G rows times the 16-byte pieces of LPR lanes:
+// the G / RPW parts of a group and the NS = b / (VEC LPR) slices of its probes
+// go to neighbouring warps, which gather the same X rows from L1 (LPR < 32:
+// several parts share a warp).  A union column costs one broadcast read of
+// its index and RPW / VEC of its values, one gather per lane and RPW x VEC
+// FMAs; U columns are in flight per warp.  The kernel is bound by the latency
+// of these gathers, which is what the parts are for: whole groups per warp
+// (16 rows x LV probes) left a 32,768-row matrix with one group per warp.
+// Measured with L2 flushed between products, us (whole groups per warp before,
+// parts now): FP32, 8-row groups, n 30,011 b 128: 47 -> 41, b 256: 76 -> 62; n
+// 65,537 b 64: 86 -> 70, b 256: 195 -> 154; 16-row groups, n 262,144 b 64: 584
+// -> 557.  Where it is used, against CSR and TMA: spmm_rule.
+template <typename VT, int RPW>
+struct RgShape {
+    static constexpr int U = 4;
+    static constexpr int MINB = (RPW * 16 <= 64) ? 3 : 2;
+};
 
-// b = 32 * LV * NS probes: NS warps share a row group, each owning a slice
-// of 32 * LV probes (LV <= 4 keeps the G x LV accumulators and two gathers in
-// flight within 128 registers, two CTAs per SM).  8 warps per CTA.
-template <typename VT, int LV, int G, int NS>
-__global__ void __launch_bounds__(256, 2)
+template <typename VT, int LPR, int RPW, bool PLAIN>
+__global__ void __launch_bounds__(256, RgShape<VT, RPW>::MINB)
 k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
-          const VT* __restrict__ gval, int64_t nrows, int64_t ngroups, int b,
+          const VT* __restrict__ gval, uint32_t nrows, uint32_t ngroups, int G, int b,
           const VT* __restrict__ X, const double* __restrict__ sx, double shift,
           VT* __restrict__ Y, const VT* __restrict__ Z, const double* __restrict__ zc,
           const double* __restrict__ zs, int epi, double* __restrict__ partials)
 {
-    __shared__ int32_t s_col[8][32];
-    __shared__ __align__(16) VT s_val[8][32][G];
-    __shared__ double s_red[8][256];
+    constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+    constexpr int RW = 32 / LPR;          // items per warp
+    constexpr int U = RgShape<VT, RPW>::U;
+    extern __shared__ double smem_rg[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int slice = warp % NS;
-    const int p0 = (slice * 32 + lane) * LV;
-    constexpr int GPC = 8 / NS;  // row groups in flight per CTA
+    const int nwarps = blockDim.x >> 5;
+    const uint32_t slices = static_cast<uint32_t>(b) / (VEC * LPR);
+    const uint32_t parts = static_cast<uint32_t>(G) / RPW;
+    // slices > 1 only where LPR = 32 (then RW = 1)
+    const int slice = warp & static_cast<int>(slices - 1);
+    const int p0 = (slice * LPR + lane % LPR) * VEC;
 
-    double sxr[LV], zcr[LV], part[LV];
+    double sxr[VEC], part[VEC];
 #pragma unroll
-    for (int v = 0; v < LV; ++v)
+    for (int v = 0; v < VEC; ++v)
     {
-        sxr[v] = sx ? sx[p0 + v] : 1.0;
-        zcr[v] = Z ? zc[p0 + v] * zs[p0 + v] : 0.0;
+        sxr[v] = pack_scale<VT, PLAIN>(sx ? sx[p0 + v] : 1.0);
         part[v] = 0.0;
     }
 
-    const int64_t gw = static_cast<int64_t>(blockIdx.x) * GPC + warp / NS;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * GPC;
-    for (int64_t g = gw; g < ngroups; g += stride)
+    const VT* Xl = X + p0;
+    const uint32_t items = ngroups * parts;
+    const uint32_t per_cta = static_cast<uint32_t>(nwarps) / slices * RW;
+    const uint32_t stride = gridDim.x * per_cta;
+    const uint32_t rs = static_cast<uint32_t>(lane) / LPR;
+    uint32_t item = blockIdx.x * per_cta + static_cast<uint32_t>(warp) / slices * RW + rs;
+    int n0 = 0, n1 = 0;
+    const int rl = lane % LPR;
+    auto prefetch_item = [&]() {
+        prefetch_l2(gcol + n0, static_cast<int64_t>(n1 - n0) * 4, rl, LPR);
+        prefetch_l2(gval + static_cast<size_t>(n0) * G,
+                    static_cast<int64_t>(n1 - n0) * G * sizeof(VT), rl, LPR);
+    };
+    if (item < items)
     {
-        VT acc[G][LV];
-#pragma unroll
-        for (int r = 0; r < G; ++r)
-#pragma unroll
-            for (int v = 0; v < LV; ++v) acc[r][v] = VT(0);
-        const int u0 = gptr[g];
-        const int u1 = gptr[g + 1];
-        for (int base = u0; base < u1; base += 32)
+        n0 = __ldg(gptr + item / parts);
+        n1 = __ldg(gptr + item / parts + 1);
+        prefetch_item();
+    }
+    for (; item < items; item += stride)
+    {
+        const uint32_t row0 = item / parts * G + item % parts * RPW;
+        const int k1 = n1;
+        int k = n0;
+        n0 = n1 = 0;
+        if (item + stride < items)
         {
-            const int cnt = min(32, u1 - base);
-            if (lane < cnt)
-            {
-                s_col[warp][lane] = __ldg(gcol + base + lane);
-                VT tmp[G];
-                ldg_n<VT, G>(gval + static_cast<int64_t>(base + lane) * G, tmp);
-                store_n<VT, G>(&s_val[warp][lane][0], tmp);
-            }
-            __syncwarp();
-            int t = 0;
-            for (; t + 2 <= cnt; t += 2)
-            {
-                const int c0 = s_col[warp][t];
-                const int c1 = s_col[warp][t + 1];
-                VT x0[LV], x1[LV];
-                ldg_n<VT, LV>(X + static_cast<int64_t>(c0) * b + p0, x0);
-                ldg_n<VT, LV>(X + static_cast<int64_t>(c1) * b + p0, x1);
-                VT a0[G], a1[G];
-                load_n<VT, G>(&s_val[warp][t][0], a0);
-                load_n<VT, G>(&s_val[warp][t + 1][0], a1);
+            n0 = __ldg(gptr + (item + stride) / parts);
+            n1 = __ldg(gptr + (item + stride) / parts + 1);
+            prefetch_item();
+        }
+        VT acc[RPW][VEC];
 #pragma unroll
-                for (int r = 0; r < G; ++r)
+        for (int r = 0; r < RPW; ++r)
 #pragma unroll
-                    for (int v = 0; v < LV; ++v)
-                    {
-                        acc[r][v] += a0[r] * x0[v];
-                        acc[r][v] += a1[r] * x1[v];
-                    }
-            }
-            if (t < cnt)
-            {
-                const int c0 = s_col[warp][t];
-                VT x0[LV];
-                ldg_n<VT, LV>(X + static_cast<int64_t>(c0) * b + p0, x0);
-                VT a0[G];
-                load_n<VT, G>(&s_val[warp][t][0], a0);
+            for (int v = 0; v < VEC; ++v) acc[r][v] = VT(0);
+        const VT* val = gval + static_cast<size_t>(k) * G + item % parts * RPW;
+        // U columns at once, their indices loaded a batch ahead
+        int nc[U];
 #pragma unroll
-                for (int r = 0; r < G; ++r)
+        for (int u = 0; u < U; ++u) nc[u] = (k + U <= k1) ? __ldg(gcol + k + u) : 0;
+        for (; k + U <= k1; k += U, val += static_cast<size_t>(U) * G)
+        {
+            VT x[U][VEC], aa[U][RPW];
 #pragma unroll
-                    for (int v = 0; v < LV; ++v) acc[r][v] += a0[r] * x0[v];
-            }
-            __syncwarp();
+            for (int u = 0; u < U; ++u) ldg_n<VT, VEC>(Xl + static_cast<size_t>(nc[u]) * b, x[u]);
+            if (k + 2 * U <= k1)
+#pragma unroll
+                for (int u = 0; u < U; ++u) nc[u] = __ldg(gcol + k + U + u);
+#pragma unroll
+            for (int u = 0; u < U; ++u) ldg_n<VT, RPW>(val + u * G, aa[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int r = 0; r < RPW; ++r)
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) acc[r][v] += aa[u][r] * x[u][v];
+        }
+#pragma unroll 1
+        for (; k < k1; ++k, val += G)
+        {
+            VT x[VEC], aa[RPW];
+            ldg_n<VT, VEC>(Xl + static_cast<size_t>(__ldg(gcol + k)) * b, x);
+            ldg_n<VT, RPW>(val, aa);
+#pragma unroll
+            for (int r = 0; r < RPW; ++r)
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) acc[r][v] += aa[r] * x[v];
         }
 #pragma unroll
-        for (int r = 0; r < G; ++r)
-        {
-            const int64_t row = g * G + r;
-            if (row < nrows)
-                spmm_row_epilogue<VT, LV>(row, b, p0, acc[r], sxr, zcr, shift, X, Y, Z, zs, epi,
-                                          part);
-        }
+        for (int r = 0; r < RPW; ++r)
+            if (row0 + r < nrows)
+                finish_piece<VT, PLAIN>(acc[r], static_cast<size_t>(row0 + r) * b + p0, p0, sxr,
+                                        sx != nullptr, shift, X, Y, Z, zc, zs, epi, part);
     }
 
     if (epi == 0) return;
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&s_red[0][0])[i] = 0.0;
-    __syncthreads();
+    // fixed order: the CTA's warps of a slice, the items of a warp
 #pragma unroll
-    for (int v = 0; v < LV; ++v) s_red[warp][p0 + v] = part[v];
+    for (int v = 0; v < VEC; ++v)
+        smem_rg[static_cast<size_t>(static_cast<uint32_t>(warp) / slices * RW + rs) * b + p0 + v] =
+            part[v];
     __syncthreads();
     for (int p = threadIdx.x; p < b; p += blockDim.x)
     {
         double s = 0.0;
-        for (int w = 0; w < 8; ++w) s += s_red[w][p];
-        partials[static_cast<int64_t>(blockIdx.x) * b + p] = s;
+        for (uint32_t w = 0; w < per_cta; ++w) s += smem_rg[static_cast<size_t>(w) * b + p];
+        const double f = epi == 1 ? (sx ? sx[p] : 1.0) : epi == 3 ? zs[p] : 1.0;
+        partials[static_cast<int64_t>(blockIdx.x) * b + p] = f * s;
     }
 }
 

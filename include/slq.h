@@ -373,9 +373,9 @@ slq_status slq_run(slq_op* op, const slq_params* p, const double* parameters,
 /* SpMM autotuner (no counterpart in the reference, whose products are one
  * cusparseSpMV per probe, cusparse_interface.cu:243).  The candidates for a
  * block width are the storage formats the operator holds crossed with their
- * tiles: CSR warp per row; row-group (the operator's group_rows rows sharing
- * a union of columns) with LV probes per lane and NS warps per row group,
- * b = 32 LV NS; in FP32 with 8- or 16-row groups at b = 128 or 256, the
+ * tiles: CSR; row-group (the operator's group_rows rows sharing a union of
+ * columns; float64: at most 8 rows) from 32 probes on, a lane holding 16
+ * bytes of probes and a warp 4 or 8 of the group's rows; in FP32 with 8- or 16-row groups at b = 128 or 256, the
  * row-group kernel whose X rows arrive by TMA gathers; and in FP32 with
  * 16-row groups at b = 128 or 256, the tensor-core row-group kernel
  * (tcgen05 kind::tf32 on TF32 hi/lo splits of both operands, accumulators
@@ -402,7 +402,7 @@ typedef struct {
                                                    /*   cores                */
     int32_t group_rows[SLQ_TUNE_MAX_CANDIDATES];
     int32_t lanes_vec[SLQ_TUNE_MAX_CANDIDATES];    /* LV probes per lane     */
-    int32_t slices[SLQ_TUNE_MAX_CANDIDATES];       /* NS warps per row group */
+    int32_t slices[SLQ_TUNE_MAX_CANDIDATES];       /* warps per row group    */
     double milliseconds[SLQ_TUNE_MAX_CANDIDATES];  /* mean per launch        */
 } slq_tune_result;
 

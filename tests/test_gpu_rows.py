@@ -107,3 +107,52 @@ def test_samples_of_wide_blocks_match_narrow_ones(cuda, width):
     a = np.asarray(wide["convergence"]["samples"][:32], float)
     b = np.asarray(narrow["convergence"]["samples"][:32], float)
     assert np.max(np.abs(a - b) / np.abs(b)) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("group_rows", [4, 8, 16])
+@pytest.mark.parametrize("n", [3, 67, 1030])
+def test_row_group_parts_equal_the_rows_product(cuda, dtype, group_rows, n):
+    """Every row-group candidate (rows per warp x slices of the probes) gives
+    the CSR product bit for bit: the same entries in the same order, the
+    padding exact zeros -- at row counts that leave the last group ragged,
+    unions around the four columns in flight, and every width."""
+    import torch
+    from imate_b200.batch import set_variant, tune_operator
+    A = _matrix(n, dtype, n + group_rows)
+    op = _DeviceOperator(A, True, True, reorder=False, aggregate=False,
+                         group_rows=group_rows)
+    for width in (32, 64, 128, 256):
+        x = np.random.default_rng(width).standard_normal((n, width)) \
+            .astype(dtype)
+        X = torch.from_numpy(x).cuda()
+        for tr in (False, True):
+            for t in (0.0, 0.5):
+                set_variant(op, width, 0, transpose=tr)
+                base = op.dot(X, transpose=tr, t=t).cpu().numpy()
+                _check((A.T if tr else A).tocsr(), x, base, t)
+                cands, _ = tune_operator(op, width, transpose=tr, reps=1)
+                for i, c in enumerate(cands):
+                    if c["kind"] == "row-group":
+                        set_variant(op, width, i, transpose=tr)
+                        got = op.dot(X, transpose=tr, t=t).cpu().numpy()
+                        assert np.array_equal(got, base), (width, tr, t, c)
+
+
+def test_row_groups_with_unaligned_buffers_fall_back(cuda):
+    import torch
+    n, width = 400, 128
+    A = _matrix(n, np.float32, 8)
+    # (slq_operator_dot itself works in the stored row order: keep A's)
+    op = _DeviceOperator(A, False, False, reorder=False, aggregate=False,
+                         group_rows=16)
+    x = np.random.default_rng(1).standard_normal((n, width)) \
+        .astype(np.float32)
+    xb = torch.zeros(n * width + 2, device="cuda")
+    yb = torch.zeros_like(xb)
+    xb[2:] = torch.from_numpy(x.reshape(-1)).cuda()
+    _lib.check(cuda.slq_operator_dot(
+        op.handle, 0, 0.0, xb[2:].data_ptr(), yb[2:].data_ptr(), width,
+        torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    _check(A, x, yb[2:].cpu().numpy().reshape(n, width), 0.0)
