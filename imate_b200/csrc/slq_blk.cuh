@@ -744,6 +744,13 @@ k_spmm_blk(const BlkArgs d)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < 4 * 256; i += NT) red[i] = 0.0;
+    if (warp == BLK_MMA)
+    {
+        tc::tmem_alloc(tmem_slot, tmem_cols);
+        tc::tmem_relinquish();
+    }
+    pdl_wait();
+    pdl_trigger();
     for (int p = tid; p < NB; p += NT)
     {
         // 2^e_p keeps every scaled |x| <= 2^14: |x| <= |x|_2 = 1 / s_p, or
@@ -773,11 +780,6 @@ k_spmm_blk(const BlkArgs d)
         c_sx[p] = static_cast<float>(ldexp(sxv, -e));
         c_ts[p] = static_cast<float>(d.shift * sxv);
         c_zcs[p] = d.Z ? static_cast<float>(d.zc[p] * d.zs[p]) : 0.0f;
-    }
-    if (warp == BLK_MMA)
-    {
-        tc::tmem_alloc(tmem_slot, tmem_cols);
-        tc::tmem_relinquish();
     }
     tc::fence_before_sync();
     __syncthreads();

@@ -1107,6 +1107,26 @@ struct Launcher {
     int64_t launches = 0;
 };
 
+// A launch that may overlap its predecessor's end (programmatic stream
+// serialization): only for kernels that call pdl_wait before they touch memory.
+template <typename... P, typename... A>
+slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                      A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    SLQ_CK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return SLQ_OK;
+}
+
 // compulsory traffic of a product: matrix once, X once, Y written once, Z
 // read once
 template <typename VT>
@@ -1127,9 +1147,8 @@ slq_status spmm_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, const 
     const size_t smem = (epi != 0) ? 8 * static_cast<size_t>(b) * sizeof(double) : 0;
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>((nrows + 7) / 8, int64_t(L.sms) * 4)));
-    k_spmm<VT, LV, KS><<<grid, 256, smem, L.st>>>(ptr, ind, vals, nrows, b, X, sx, shift, Y, Z,
-                                                  zc, zs, epi, partials);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_spmm<VT, LV, KS>, grid, 256, smem, ptr, ind, vals, nrows, b, X, sx,
+                       shift, Y, Z, zc, zs, epi, partials));
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -1170,9 +1189,9 @@ slq_status spmm_rows_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, c
     const int64_t want = (nrows + RW * warps - 1) / (RW * warps);
     const int grid =
         static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(L.sms) * per_sm)));
-    k_spmm_rows<VT, LPR, C, PLAIN><<<grid, warps * 32, epi != 0 ? smem_of(warps) : 0, L.st>>>(
-        ptr, ind, vals, static_cast<uint32_t>(nrows), X, sx, shift, Y, Z, zc, zs, epi, partials);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_spmm_rows<VT, LPR, C, PLAIN>, grid, warps * 32,
+                       epi != 0 ? smem_of(warps) : 0, ptr, ind, vals, nrows, X, sx, shift, Y, Z, zc,
+                       zs, epi, partials));
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -1244,12 +1263,15 @@ slq_status finalize(Launcher& L, const double* partials, int nparts, int cols, i
                     double* next_scale, int32_t* active, int32_t* size, int check_break,
                     double thr, int step)
 {
-    const int grid = (cols + 31) / 32;
     ProfScope prof(SLQ_K_FINALIZE, double(nparts) * cols * 8.0, L.st);
-    k_finalize<VT><<<grid, 1024, 0, L.st>>>(partials, nparts, cols, mode, out, coef, scales, b,
-                                           bs, last, next_scale, active, size, check_break, thr,
-                                           step);
-    SLQ_LAUNCH_CK();
+    if (mode == FIN_COEF)
+        SLQ_TRY(launch_pdl(L.st, k_finalize<VT, 32, 32>, (cols + 31) / 32, 1024, 0, partials, nparts,
+                           cols, mode, out, coef, scales, b, bs, last, next_scale, active, size,
+                           check_break, thr, step));
+    else
+        SLQ_TRY(launch_pdl(L.st, k_finalize<VT, 8, 64>, (cols + 7) / 8, 512, 0, partials, nparts,
+                           cols, mode, out, coef, scales, b, bs, last, next_scale, active, size,
+                           check_break, thr, step));
     ++L.launches;
     return SLQ_OK;
 }
@@ -1541,10 +1563,8 @@ slq_status spmm_rg_inst(Launcher& L, const int32_t* gptr, const int32_t* gcol, c
     const size_t smem = epi != 0 ? static_cast<size_t>(per_cta) * b * sizeof(double) : 0;
     const int grid = static_cast<int>(std::max<int64_t>(
         1, std::min<int64_t>((items + per_cta - 1) / per_cta, int64_t(L.sms) * per_sm)));
-    k_spmm_rg<VT, LPR, RPW, PLAIN><<<grid, warps * 32, smem, L.st>>>(
-        gptr, gcol, gval, static_cast<uint32_t>(nrows), static_cast<uint32_t>(ng), G, b, X, sx,
-        shift, Y, Z, zc, zs, epi, partials);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_spmm_rg<VT, LPR, RPW, PLAIN>, grid, warps * 32, smem, gptr, gcol,
+                       gval, nrows, ng, G, b, X, sx, shift, Y, Z, zc, zs, epi, partials));
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -1690,14 +1710,13 @@ slq_status spmm_blk_inst(Launcher& L, const slq_op* op, int transpose, int b, co
     d.x16 = pre ? maps->x16 : nullptr;
     d.xexp = ready ? maps->x16exp : nullptr;
     if (pre && b == 256)
-        k_spmm_blk<256, true><<<grid, BLK_THREADS, smem, L.st>>>(d);
+        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<256, true>, grid, BLK_THREADS, smem, d));
     else if (pre)
-        k_spmm_blk<128, true><<<grid, BLK_THREADS, smem, L.st>>>(d);
+        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<128, true>, grid, BLK_THREADS, smem, d));
     else if (b == 256)
-        k_spmm_blk<256, false><<<grid, BLK_THREADS, smem, L.st>>>(d);
+        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<256, false>, grid, BLK_THREADS, smem, d));
     else
-        k_spmm_blk<128, false><<<grid, BLK_THREADS, smem, L.st>>>(d);
-    SLQ_LAUNCH_CK();
+        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<128, false>, grid, BLK_THREADS, smem, d));
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -1984,8 +2003,7 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     // the split parts: 2 x 2 bytes per element, one float vector's bytes
     const int writes = ((MODE == 1 || do_update) ? 1 : 0) + (x16 ? 1 : 0);
     ProfScope prof(MODE == 0 ? SLQ_K_DOTS : SLQ_K_REORTH, vb * (reads + writes), L.st);
-    k_stream<VT, MODE, R><<<dim3(gx, gy), STREAM_THREADS, smem, L.st>>>(a);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_stream<VT, MODE, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
     ++L.launches;
     *grid_out = gx;
     return SLQ_OK;
@@ -2170,16 +2188,14 @@ slq_status launch_quadrature(Launcher& L, const RunPlan& r, const slq_params* p,
                              int count, double* samples, int32_t* status)
 {
     ProfScope prof(SLQ_K_EIG, double(r.m) * r.b * 16.0 + double(count) * r.q * 8.0, L.st);
-    k_ql<<<count, 32, 3 * sizeof(double) * r.m, L.st>>>(r.b, r.m, B.alpha, B.beta, B.size,
-                                                        r.gram == 1, B.theta, B.tau, status);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_ql, count, 32, 3 * sizeof(double) * r.m, r.b, r.m, B.alpha, B.beta,
+                       B.size, r.gram == 1, B.theta, B.tau, status));
     ++L.launches;
     const int64_t pairs = int64_t(count) * r.q;
     const int grid = static_cast<int>(std::min<int64_t>((pairs + 7) / 8, int64_t(L.sms) * 8));
-    k_quad<<<grid, 256, 0, L.st>>>(count, r.b, r.m, B.size, B.theta, B.tau, p->func,
-                                   func_coeff(p), p->exponent, B.params, r.q,
-                                   static_cast<double>(r.nv), samples, status);
-    SLQ_LAUNCH_CK();
+    SLQ_TRY(launch_pdl(L.st, k_quad, grid, 256, 0, count, r.b, r.m, B.size, B.theta, B.tau, p->func,
+                       func_coeff(p), p->exponent, B.params, r.q, static_cast<double>(r.nv), samples,
+                       status));
     ++L.launches;
     return SLQ_OK;
 }

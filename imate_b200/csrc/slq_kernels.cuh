@@ -134,6 +134,18 @@ __device__ __forceinline__ void store_n(VT* p, const VT (&v)[N])
     }
 }
 
+// Programmatic dependent launch (the kernels of a Krylov step, launched with
+// launch_pdl): a kernel may become resident while its predecessor runs, and
+// waits here, before its first access to memory, until the predecessor has
+// completed and its writes are visible.  Since each one waits, a kernel's
+// completion implies that of all before it.  Without the launch attribute
+// both are no-ops.  What it saves is the launch gap between small kernels.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 
 __device__ __forceinline__ int ring_slot(int vec, int bs)
@@ -179,6 +191,8 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
 {
     constexpr int P = 32 / KS;
     extern __shared__ double smem_spmm[];
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
@@ -466,6 +480,8 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
     constexpr int U = SpmmRowsShape<VT, C>::U;
     constexpr int LV = C * VEC;
     extern __shared__ double smem_rows[];
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
@@ -599,32 +615,55 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
 //               : 0; with check_break, probes whose nrm < thr stop at size
 //               step+1 (the breakdown test of c_lanczos_tridiagonalization
 //               .cpp:225-228).
-// 32 x 32 threads: 32 columns per CTA, 32 partial rows per column.
+// CW columns per CTA, RL threads per column, each summing every RL-th partial
+// row with four loads in flight; a warp per column adds the RL sums.  The
+// kernel is a chain of a few L2 reads, so few columns (alpha, norms: b of
+// them) take narrow CTAs with more threads per column.  With its launch overlapped
+// (pdl_wait) a step of small matrices lost 2.3 us per launch: a 500-row
+// degree-20 call of 84 launches 1.25 -> 1.05 ms.
 // ---------------------------------------------------------------------------
 
 enum { FIN_STORE = 0, FIN_COEF = 1, FIN_NORM = 2 };
 
-template <typename VT>
-__global__ void __launch_bounds__(1024)
+template <typename VT, int CW, int RL>
+__global__ void __launch_bounds__(CW * RL)
 k_finalize(const double* __restrict__ partials, int nparts, int cols, int mode,
            double* __restrict__ out, VT* __restrict__ coef,
            const double* __restrict__ scales, int b, int bs, int last,
            double* __restrict__ next_scale, int32_t* __restrict__ active,
            int32_t* __restrict__ size, int check_break, double thr, int step)
 {
-    __shared__ double red[32][33];
-    const int cx = threadIdx.x & 31;
-    const int cy = threadIdx.x >> 5;
-    const int col = blockIdx.x * 32 + cx;
-    double s = 0.0;
-    if (col < cols)
-        for (int q = cy; q < nparts; q += 32)
-            s += partials[static_cast<int64_t>(q) * cols + col];
-    red[cy][cx] = s;
+    __shared__ double red[RL][CW + 1];
+    pdl_wait();
+    pdl_trigger();
+    const int cx = threadIdx.x % CW;
+    const int cy = threadIdx.x / CW;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (blockIdx.x * CW + cx < cols)
+    {
+        const double* p = partials + blockIdx.x * CW + cx;
+        int q = cy;
+        for (; q + 3 * RL < nparts; q += 4 * RL)
+        {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[u] += p[static_cast<int64_t>(q + u * RL) * cols];
+        }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (q + u * RL < nparts) acc[u] += p[static_cast<int64_t>(q + u * RL) * cols];
+    }
+    red[cy][cx] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     __syncthreads();
-    if (cy != 0 || col >= cols) return;
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int col = blockIdx.x * CW + w;
+    if (w >= CW || col >= cols) return;
     double t = 0.0;
-    for (int q = 0; q < 32; ++q) t += red[q][cx];
+#pragma unroll
+    for (int r = 0; r < RL; r += 32) t += red[r + lane][w];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(FULL_MASK, t, off);
+    if (lane != 0) return;
 
     if (mode == FIN_STORE)
     {
@@ -812,6 +851,8 @@ k_ql(int b, int m, const double* __restrict__ alpha, const double* __restrict__ 
      double* __restrict__ tau, int32_t* __restrict__ status)
 {
     extern __shared__ double smem_ql[];
+    pdl_wait();
+    pdl_trigger();
     double* d = smem_ql;
     double* e = d + m;
     double* z = e + m;
@@ -859,6 +900,8 @@ k_quad(int count, int b, int m, const int32_t* __restrict__ size,
        double exponent, const double* __restrict__ params, int q, double nscale,
        double* __restrict__ samples, int32_t* __restrict__ status)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const double t0 = params[0];
     const int64_t pairs = static_cast<int64_t>(count) * q;
@@ -1902,10 +1945,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (MODE == 0)
-    {
         for (int i = tid; i < J * STREAM_CONSUMERS; i += STREAM_THREADS) extra[i] = 0.0;
-    }
-    else
+    pdl_wait();
+    pdl_trigger();
+    if (MODE == 1)
     {
         for (int i = tid; i < J * PT; i += STREAM_THREADS)
             extra[i] = static_cast<double>(a.coef[static_cast<int64_t>(i / PT) * b + p0 + i % PT]);
@@ -2351,6 +2394,8 @@ k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
     constexpr int RW = 32 / LPR;          // items per warp
     constexpr int U = RgShape<VT, RPW>::U;
     extern __shared__ double smem_rg[];
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
