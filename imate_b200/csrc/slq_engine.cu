@@ -2063,6 +2063,43 @@ int buffer_size(int gram, int orth, int m)
     return orth;
 }
 
+// Words per chunk of a probe of wpp words: short probes in one piece (no
+// jumps), else pieces that give every SM some, at most `most` of them.
+void plan_chunks(RunPlan* r, int64_t most)
+{
+    r->cw = r->wpp <= 64 ? 64 : PROBE_WORDS;
+    while ((r->wpp + r->cw - 1) / r->cw > most) r->cw *= 2;
+    r->nchunks = static_cast<int>((r->wpp + r->cw - 1) / r->cw);
+}
+
+// Words of the two jump tables of a sequence of n entries.
+size_t jump_table_words(int64_t n)
+{
+    return static_cast<size_t>(PROBE_FAN + (n + PROBE_FAN - 1) / PROBE_FAN) * 4;
+}
+
+// The two tables of x^(i d) mod P, i < n, given step = x^d mod P, into
+// out[jump_table_words(n)].
+void jump_tables(const Poly256& step, int64_t n, uint64_t* out)
+{
+    Poly256 acc = {{1, 0, 0, 0}};
+    auto put = [&]() {
+        for (int k = 0; k < 4; ++k) *out++ = acc.w[k];
+    };
+    for (int i = 0; i < PROBE_FAN; ++i)
+    {
+        put();
+        acc = poly_mulmod(acc, step);
+    }
+    const Poly256 wide = acc;  // x^(PROBE_FAN d)
+    acc = {{1, 0, 0, 0}};
+    for (int64_t i = 0; i * PROBE_FAN < n; ++i)
+    {
+        put();
+        if ((i + 1) * PROBE_FAN < n) acc = poly_mulmod(acc, wide);
+    }
+}
+
 slq_status make_plan(const slq_op* op, const slq_params* p, int q, RunPlan* r)
 {
     if (!op || !p) return fail(SLQ_ERR_BAD_ARG, "NULL operator or params");
@@ -2110,9 +2147,7 @@ slq_status make_plan(const slq_op* op, const slq_params* p, int q, RunPlan* r)
     r->x16 = op->dtype == SLQ_F32 && !op->dense && op->a_nblk > 0 && r->gram != 1 &&
              (b == 128 || b == 256);
     r->wpp = r->nv / 64 + 1;
-    r->cw = 64;
-    while ((r->wpp + r->cw - 1) / r->cw > 65535) r->cw *= 2;
-    r->nchunks = static_cast<int>((r->wpp + r->cw - 1) / r->cw);
+    plan_chunks(r, 65535);
     return SLQ_OK;
 }
 
@@ -2157,7 +2192,7 @@ void carve(Carver& c, const RunPlan& r, int sms, RunBufs* B)
     B->samples = c.take<double>(static_cast<size_t>(r.b) * r.q);
     B->params = c.take<double>(r.q);
     B->starts = c.take<uint64_t>(static_cast<size_t>(r.b) * 4);
-    B->chunk_polys = c.take<uint64_t>(static_cast<size_t>(r.nchunks) * 4);
+    B->chunk_polys = c.take<uint64_t>(jump_table_words(r.nchunks) + jump_table_words(r.b));
 }
 
 double4 func_coeff(const slq_params* p)
@@ -2169,16 +2204,22 @@ template <typename VT>
 slq_status launch_probes(Launcher& L, const RunPlan& r, int rng, int64_t seed, int64_t first,
                          int count, const RunBufs& B, const int32_t* inv, VT* X)
 {
-    dim3 grid((r.b + 127) / 128, r.nchunks);
     ProfScope prof(SLQ_K_PROBE, double(r.nv) * r.b * sizeof(VT), L.st);
     if (rng == SLQ_RNG_PARITY)
-        k_probe_parity<VT><<<grid, 128, 0, L.st>>>(r.nv, r.b, count, r.wpp, r.cw, B.starts,
-                                                   B.chunk_polys, inv, X);
+    {
+        const dim3 grid(static_cast<unsigned>((r.b + PROBE_TILE - 1) / PROBE_TILE),
+                        static_cast<unsigned>(r.nchunks));
+        SLQ_TRY(launch_pdl(L.st, k_probe_parity<VT>, grid, 256, 0, r.nv, r.b, count, r.wpp, r.cw,
+                           B.starts, B.chunk_polys, B.chunk_polys + PROBE_FAN * 4, inv, X));
+    }
     else
+    {
+        const dim3 grid((r.b + 127) / 128, r.nchunks);
         k_probe_fast<VT><<<grid, 128, 0, L.st>>>(r.nv, r.b, count, first,
                                                  static_cast<uint64_t>(seed) * 0xd1342543de82ef95ULL,
                                                  r.wpp, r.cw, inv, X);
-    SLQ_LAUNCH_CK();
+        SLQ_LAUNCH_CK();
+    }
     ++L.launches;
     return SLQ_OK;
 }
@@ -2412,7 +2453,8 @@ slq_status krylov_block(Launcher& L, const slq_op* op, const slq_params* p, cons
 }
 
 // Parity stream set-up of a run: start state of its probe 0, the advance
-// polynomial between consecutive probes and the per-chunk polynomials.
+// polynomial between consecutive probes, and the jump tables of the chunks
+// followed by those of a block's probes.
 slq_status parity_setup(const slq_params* p, const RunPlan& r, uint64_t* cur, Poly256* advance,
                         std::vector<uint64_t>* polys)
 {
@@ -2420,14 +2462,9 @@ slq_status parity_setup(const slq_params* p, const RunPlan& r, uint64_t* cur, Po
     stream_state(p->seed, cur);
     jump_ahead(cur, static_cast<uint64_t>(p->first_probe) * static_cast<uint64_t>(r.wpp));
     *advance = jump_poly(static_cast<uint64_t>(r.wpp));
-    polys->assign(static_cast<size_t>(r.nchunks) * 4, 0);
-    const Poly256 step = jump_poly(static_cast<uint64_t>(r.cw));
-    Poly256 acc = {{1, 0, 0, 0}};
-    for (int cidx = 0; cidx < r.nchunks; ++cidx)
-    {
-        for (int k = 0; k < 4; ++k) (*polys)[static_cast<size_t>(cidx) * 4 + k] = acc.w[k];
-        acc = poly_mulmod(acc, step);
-    }
+    polys->resize(jump_table_words(r.nchunks) + jump_table_words(r.b));
+    jump_tables(jump_poly(static_cast<uint64_t>(r.cw)), r.nchunks, polys->data());
+    jump_tables(*advance, r.b, polys->data() + jump_table_words(r.nchunks));
     return SLQ_OK;
 }
 
@@ -2506,7 +2543,6 @@ slq_status run_typed(slq_op* op, const slq_params* p, const double* parameters, 
         ha.resize(static_cast<size_t>(m) * b);
         hb.resize(static_cast<size_t>(m) * b);
     }
-    std::vector<uint64_t> hstarts(static_cast<size_t>(b) * 4);
     const double s0 = 1.0 / std::sqrt(static_cast<double>(r.nv));
     int nproc = 0;
     int all = 0;
@@ -2519,14 +2555,20 @@ slq_status run_typed(slq_op* op, const slq_params* p, const double* parameters, 
         const int count = std::min(b, max_s - g);
         if (p->rng == SLQ_RNG_PARITY)
         {
-            for (int pi = 0; pi < count; ++pi)
+            // the probes' start states on the device; the host moves on by
+            // the block
+            const uint64_t* adv = B.chunk_polys + jump_table_words(r.nchunks);
+            const ulonglong4 s0v = make_ulonglong4(cur[0], cur[1], cur[2], cur[3]);
+            SLQ_TRY(launch_pdl(st, k_probe_starts, (count + 31) / 32, 32, 0, count, s0v, adv,
+                               adv + PROBE_FAN * 4, B.starts));
+            ++L.launches;
+            if (g + b < max_s)
             {
-                for (int k = 0; k < 4; ++k) hstarts[static_cast<size_t>(pi) * 4 + k] = cur[k];
+                if (g == 0)
+                    // x^(b wpp): b is a power of two
+                    for (int w = 1; w < b; w *= 2) advance = poly_mulmod(advance, advance);
                 apply_poly(advance, cur);
             }
-            SLQ_CK(cudaMemcpyAsync(B.starts, hstarts.data(),
-                                   sizeof(uint64_t) * 4 * static_cast<size_t>(count),
-                                   cudaMemcpyHostToDevice, st));
         }
         SLQ_TRY(launch_probes<VT>(L, r, p->rng, p->seed, p->first_probe + g, count, B,
                                   op->inv, static_cast<VT*>(B.V)));
@@ -3596,13 +3638,12 @@ extern "C" slq_status slq_generate_probes_workspace_bytes(int64_t len, int width
                                                           size_t* bytes)
 {
     if (!bytes || len <= 0 || width <= 0) return fail(SLQ_ERR_BAD_ARG, "bad argument");
-    const int64_t wpp = len / 64 + 1;
-    int cw = 64;
-    while ((wpp + cw - 1) / cw > 65535) cw *= 2;
-    const int64_t nchunks = (wpp + cw - 1) / cw;
+    RunPlan r;
+    r.wpp = len / 64 + 1;
+    plan_chunks(&r, 65535);
     Carver c(nullptr, 0);
     c.take<uint64_t>(static_cast<size_t>(width) * 4);
-    c.take<uint64_t>(static_cast<size_t>(nchunks) * 4);
+    c.take<uint64_t>(jump_table_words(r.nchunks));
     *bytes = c.off + 256;
     return SLQ_OK;
 }
@@ -3623,13 +3664,11 @@ extern "C" slq_status slq_generate_probes(int64_t seed, int rng, int64_t len, in
     r.nv = len;
     r.b = width;
     r.wpp = len / 64 + 1;
-    r.cw = 64;
-    while ((r.wpp + r.cw - 1) / r.cw > 65535) r.cw *= 2;
-    r.nchunks = static_cast<int>((r.wpp + r.cw - 1) / r.cw);
+    plan_chunks(&r, 65535);
     Carver c(workspace, workspace_bytes);
     RunBufs B;
     B.starts = c.take<uint64_t>(static_cast<size_t>(width) * 4);
-    B.chunk_polys = c.take<uint64_t>(static_cast<size_t>(r.nchunks) * 4);
+    B.chunk_polys = c.take<uint64_t>(jump_table_words(r.nchunks));
     if (rng == SLQ_RNG_PARITY)
     {
         if (!self_check()) return fail(SLQ_ERR_CUDA, "jump polynomial self-check failed");
@@ -3643,14 +3682,8 @@ extern "C" slq_status slq_generate_probes(int64_t seed, int rng, int64_t len, in
             for (int k = 0; k < 4; ++k) hs[static_cast<size_t>(pi) * 4 + k] = cur[k];
             apply_poly(adv, cur);
         }
-        std::vector<uint64_t> polys(static_cast<size_t>(r.nchunks) * 4);
-        const Poly256 step = jump_poly(static_cast<uint64_t>(r.cw));
-        Poly256 acc = {{1, 0, 0, 0}};
-        for (int ci = 0; ci < r.nchunks; ++ci)
-        {
-            for (int k = 0; k < 4; ++k) polys[static_cast<size_t>(ci) * 4 + k] = acc.w[k];
-            acc = poly_mulmod(acc, step);
-        }
+        std::vector<uint64_t> polys(jump_table_words(r.nchunks));
+        jump_tables(jump_poly(static_cast<uint64_t>(r.cw)), r.nchunks, polys.data());
         SLQ_CK(cudaMemcpyAsync(B.starts, hs.data(), hs.size() * 8, cudaMemcpyHostToDevice, st));
         SLQ_CK(cudaMemcpyAsync(B.chunk_polys, polys.data(), polys.size() * 8,
                                cudaMemcpyHostToDevice, st));
@@ -3750,9 +3783,10 @@ extern "C" slq_status slq_generate_probes_noalloc(int64_t seed, int rng, int64_t
     r.nv = len;
     r.b = width;
     r.wpp = len / 64 + 1;
-    r.cw = 64;
-    while ((r.wpp + r.cw - 1) / r.cw > NOALLOC_MAX_CHUNKS) r.cw *= 2;
-    r.nchunks = static_cast<int>((r.wpp + r.cw - 1) / r.cw);
+    // the two tables of at most NOALLOC_MAX_CHUNKS chunks fit the scratch
+    plan_chunks(&r, NOALLOC_MAX_CHUNKS);
+    static_assert(PROBE_FAN + NOALLOC_MAX_CHUNKS / PROBE_FAN <= NOALLOC_MAX_CHUNKS,
+                  "jump tables larger than the scratch");
     RunBufs B;
     B.starts = scratch;
     B.chunk_polys = scratch + static_cast<size_t>(NOALLOC_MAX_WIDTH) * 4;
@@ -3770,17 +3804,11 @@ extern "C" slq_status slq_generate_probes_noalloc(int64_t seed, int rng, int64_t
             for (int k = 0; k < 4; ++k) hs[static_cast<size_t>(pi) * 4 + k] = cur[k];
             apply_poly(adv, cur);
         }
-        const Poly256 step = jump_poly(static_cast<uint64_t>(r.cw));
-        Poly256 acc = {{1, 0, 0, 0}};
-        for (int ci = 0; ci < r.nchunks; ++ci)
-        {
-            for (int k = 0; k < 4; ++k) hp[static_cast<size_t>(ci) * 4 + k] = acc.w[k];
-            acc = poly_mulmod(acc, step);
-        }
+        jump_tables(jump_poly(static_cast<uint64_t>(r.cw)), r.nchunks, hp);
         SLQ_CK(cudaMemcpyAsync(B.starts, hs, sizeof(uint64_t) * 4 * static_cast<size_t>(count),
                                cudaMemcpyHostToDevice, st));
         SLQ_CK(cudaMemcpyAsync(B.chunk_polys, hp,
-                               sizeof(uint64_t) * 4 * static_cast<size_t>(r.nchunks),
+                               sizeof(uint64_t) * jump_table_words(r.nchunks),
                                cudaMemcpyHostToDevice, st));
         // the host staging is reused by the next call
         SLQ_CK(cudaStreamSynchronize(st));
