@@ -1942,25 +1942,29 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
                        double* wn2_out = nullptr, const double* wn2_in = nullptr,
                        int wn2_grid = 0, __half* x16 = nullptr, int32_t* x16exp = nullptr)
 {
+    // rows per consumer thread: 16 KB tiles (half of that took nearly the
+    // same time per tile: the consumers' latency, not the bytes)
     constexpr int R = (sizeof(VT) == 4) ? 16 : 8;
     constexpr size_t SMEM_MAX = 232448;
+    constexpr size_t TILE = static_cast<size_t>(R) * STREAM_CONSUMERS * sizeof(VT);
     const int PT = std::min(b, STREAM_CONSUMERS);
     const int T = R * (STREAM_CONSUMERS / PT);
-    const size_t fixed = 256 + STREAM_CONSUMERS * sizeof(double);
+    const size_t fixed = STREAM_BARRIER_BYTES + STREAM_CONSUMERS * sizeof(double);
     const size_t extra = (MODE == 0) ? static_cast<size_t>(J) * STREAM_CONSUMERS * 8
                                      : static_cast<size_t>(J) * PT * 8;
-    if (fixed + extra + 2 * STREAM_TILE_BYTES > SMEM_MAX)
+    if (fixed + extra + 2 * TILE > SMEM_MAX)
         return fail(SLQ_ERR_BAD_ARG, "stream pass: too many basis vectors per launch");
-    const int S = static_cast<int>(std::min<size_t>(STREAM_MAX_STAGES,
-                                                    (SMEM_MAX - fixed - extra) / STREAM_TILE_BYTES));
-    const size_t smem = fixed + static_cast<size_t>(S) * STREAM_TILE_BYTES + extra;
-    static bool attr = false;
-    if (!attr)
+    const int S = static_cast<int>(std::min<size_t>(STREAM_RING_BYTES / TILE,
+                                                    (SMEM_MAX - fixed - extra) / TILE));
+    const size_t smem = fixed + static_cast<size_t>(S) * TILE + extra;
+    auto kernel = (MODE == 1 && J == 0) ? k_stream<VT, MODE, R, false>
+                                        : k_stream<VT, MODE, R, MODE == 1>;
+    static bool attr[2] = {false, false};
+    if (!attr[J == 0])
     {
-        SLQ_CK(cudaFuncSetAttribute(k_stream<VT, MODE, R>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+        SLQ_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(SMEM_MAX)));
-        attr = true;
+        attr[J == 0] = true;
     }
     StreamArgs<VT> a;
     a.n = n;
@@ -2003,7 +2007,7 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     // the split parts: 2 x 2 bytes per element, one float vector's bytes
     const int writes = ((MODE == 1 || do_update) ? 1 : 0) + (x16 ? 1 : 0);
     ProfScope prof(MODE == 0 ? SLQ_K_DOTS : SLQ_K_REORTH, vb * (reads + writes), L.st);
-    SLQ_TRY(launch_pdl(L.st, k_stream<VT, MODE, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
+    SLQ_TRY(launch_pdl(L.st, kernel, dim3(gx, gy), STREAM_THREADS, smem, a));
     ++L.launches;
     *grid_out = gx;
     return SLQ_OK;

@@ -1827,7 +1827,9 @@ __global__ void k_init_block(int count, int b, int m, double s0,
 //            <v_i, w> per (i, probe);
 //   reorth : Win, then the basis vectors last-i: w -= c_i v_i, written to
 //            Wout, FP64 partials of |w|^2.
-// Rows past the last whole tile are done by the last CTA with plain loads.
+// Rows past the last whole tile are dealt over the CTAs with plain loads (one
+// CTA alone took 20 us for the 27 rows past 937 tiles of a 30,011-row matrix,
+// as long as the tiles took the others).
 //
 // Every mbarrier wait is bounded; a wait that runs out sets *error and the
 // CTA skips the remaining work (it still waits, bounded, for the copies it
@@ -1836,8 +1838,9 @@ __global__ void k_init_block(int count, int b, int m, double s0,
 
 constexpr int STREAM_CONSUMERS = 256;            // 8 consumer warps
 constexpr int STREAM_THREADS = STREAM_CONSUMERS + 32;
-constexpr int STREAM_TILE_BYTES = 16384;
-constexpr int STREAM_MAX_STAGES = 8;
+constexpr int STREAM_MAX_STAGES = 16;
+constexpr int STREAM_RING_BYTES = 131072;  // copies in flight per CTA
+constexpr int STREAM_BARRIER_BYTES = 2 * STREAM_MAX_STAGES * 8 + 64;
 constexpr long long STREAM_SPIN_LIMIT = 1LL << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
@@ -1976,20 +1979,22 @@ struct StreamArgs {
 };
 
 // MODE 0: dots, MODE 1: reorth.  R = rows per consumer thread per tile.
-template <typename VT, int MODE, int R>
+// PAIR: MODE 1 takes two basis tiles per turn; without basis vectors (J = 0,
+// the plain three-term update) the code for it only costs (524,175 x 256 FP32:
+// 346 us without it, 372 with).
+template <typename VT, int MODE, int R, bool PAIR>
 __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<VT> a)
 {
-    // shared memory: barriers (256 B) | norm partials (256 doubles) |
-    // S stages of 16 KB | dots: acc[J][256] doubles, reorth: coef[J][PT]
+    // shared memory: barriers | norm partials (256 doubles) | S stages of
+    // R x 256 values | dots: acc[J][256] doubles, reorth: coef[J][PT]
     extern __shared__ __align__(128) unsigned char smem_stream[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_stream);
     uint64_t* empty = full + STREAM_MAX_STAGES;
     int* abort_flag = reinterpret_cast<int*>(empty + STREAM_MAX_STAGES);
-    double* red = reinterpret_cast<double*>(smem_stream + 256);
-    VT* stages = reinterpret_cast<VT*>(smem_stream + 256 + STREAM_CONSUMERS * 8);
-    const int tile_elems = a.T * a.PT;
-    double* extra = reinterpret_cast<double*>(smem_stream + 256 + STREAM_CONSUMERS * 8 +
-                                              static_cast<size_t>(a.S) * STREAM_TILE_BYTES);
+    constexpr int TILE = R * STREAM_CONSUMERS;  // values of a tile: T rows x PT probes
+    double* red = reinterpret_cast<double*>(smem_stream + STREAM_BARRIER_BYTES);
+    VT* stages = reinterpret_cast<VT*>(red + STREAM_CONSUMERS);
+    double* extra = reinterpret_cast<double*>(stages + static_cast<size_t>(a.S) * TILE);
 
     const int tid = threadIdx.x;
     const bool producer = tid >= STREAM_CONSUMERS;
@@ -2033,7 +2038,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
 
     const int64_t ntiles = a.n / a.T;
     const bool contiguous = (PT == b);
-    const uint32_t tile_bytes = static_cast<uint32_t>(tile_elems * sizeof(VT));
+    constexpr uint32_t tile_bytes = TILE * sizeof(VT);
     auto item_ptr = [&](int item) -> const VT* {
         if (item == 0) return a.W;
         if (upd && item == 1) return a.Vj;
@@ -2063,7 +2068,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                         ok = false;
                         break;
                     }
-                    VT* dst = stages + static_cast<size_t>(s) * (STREAM_TILE_BYTES / sizeof(VT));
+                    VT* dst = stages + static_cast<size_t>(s) * TILE;
                     const VT* src = item_ptr(item) + row0 * b + p0;
                     mbar_expect_tx(&full[s], tile_bytes);
                     if (contiguous)
@@ -2155,8 +2160,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                         ok = false;
                         break;
                     }
-                    const VT* t0 = stages + static_cast<size_t>(s) * (STREAM_TILE_BYTES / sizeof(VT));
-                    const VT* t1 = stages + static_cast<size_t>(s1) * (STREAM_TILE_BYTES / sizeof(VT));
+                    const VT* t0 = stages + static_cast<size_t>(s) * TILE;
+                    const VT* t1 = stages + static_cast<size_t>(s1) * TILE;
                     double l0[4] = {0.0, 0.0, 0.0, 0.0}, l1[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
                     for (int k = 0; k < R; ++k)
@@ -2168,6 +2173,42 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                     extra[ib * STREAM_CONSUMERS + tid] = prev0 + ((l0[0] + l0[1]) + (l0[2] + l0[3]));
                     extra[(ib + 1) * STREAM_CONSUMERS + tid] =
                         prev1 + ((l1[0] + l1[1]) + (l1[2] + l1[3]));
+                    release(s);
+                    release(s1);
+                    s = s1 + 1;
+                    phase = ph1;
+                    if (s == a.S) { s = 0; phase ^= 1; }
+                    ++item;
+                    continue;
+                }
+                if (MODE == 1 && PAIR && item >= npre && item + 1 < nitems)
+                {
+                    // reorth: two basis tiles per turn as well, so that their
+                    // loads and conversions overlap (262,144 x 256 FP32,
+                    // J = 25: 1,252 -> 1,197 us)
+                    const int ib = skip + (item - npre);
+                    const double c0 = extra[ib * PT + pl];
+                    const double c1 = extra[(ib + 1) * PT + pl];
+                    int s1 = s + 1;
+                    uint32_t ph1 = phase;
+                    if (s1 == a.S) { s1 = 0; ph1 ^= 1; }
+                    if (!mbar_wait(&full[s], phase, abort_flag) ||
+                        !mbar_wait(&full[s1], ph1, abort_flag))
+                    {
+                        *abort_flag = 1;
+                        atomicExch(a.error, 1);
+                        ok = false;
+                        break;
+                    }
+                    const VT* t0 = stages + static_cast<size_t>(s) * TILE;
+                    const VT* t1 = stages + static_cast<size_t>(s1) * TILE;
+#pragma unroll
+                    for (int k = 0; k < R; ++k)
+                    {
+                        const int e = (roff + k * RSTEP) * PT + pl;
+                        w[k] -= c0 * static_cast<double>(t0[e]);
+                        w[k] -= c1 * static_cast<double>(t1[e]);
+                    }
                     release(s);
                     release(s1);
                     s = s1 + 1;
@@ -2191,7 +2232,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                     ok = false;
                     break;
                 }
-                const VT* st = stages + static_cast<size_t>(s) * (STREAM_TILE_BYTES / sizeof(VT));
+                const VT* st = stages + static_cast<size_t>(s) * TILE;
                 if (item == 0)
                 {
 #pragma unroll
@@ -2275,11 +2316,13 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
             }
         }
 
-        // rows past the last whole tile: plain loads, last CTA only
+        // rows past the last whole tile: plain loads, from the last CTA back
+        // (the first ones have a tile more)
         const int64_t tail0 = ntiles * a.T;
-        if (ok && blockIdx.x == gridDim.x - 1 && tail0 < a.n)
+        if (ok)
         {
-            for (int64_t r = tail0 + roff; r < a.n; r += RSTEP)
+            const int64_t from = static_cast<int64_t>(gridDim.x - 1 - blockIdx.x) * RSTEP + roff;
+            for (int64_t r = tail0 + from; r < a.n; r += static_cast<int64_t>(gridDim.x) * RSTEP)
             {
                 const int64_t o = r * b + p0 + pl;
                 double wv = static_cast<double>(a.W[o]);
@@ -2303,6 +2346,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                         if (a.Vm && J > 1) extra[STREAM_CONSUMERS + tid] += y * wv;
                     }
                 }
+#pragma unroll 4
                 for (int i = skip; i < J; ++i)
                 {
                     const VT* vp = a.basis + static_cast<int64_t>(ring_slot(a.last - i, a.bs)) * a.slot_elems;
