@@ -2037,6 +2037,12 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
     __syncthreads();
 
     const int64_t ntiles = a.n / a.T;
+    // MODE 1 walks the tiles backwards: it starts on what the pass (or product)
+    // before it read and wrote last, which is still in L2, and ends where the
+    // next product starts
+    auto first_row = [&](int64_t tile) {
+        return (MODE == 1 ? ntiles - 1 - tile : tile) * a.T;
+    };
     const bool contiguous = (PT == b);
     constexpr uint32_t tile_bytes = TILE * sizeof(VT);
     auto item_ptr = [&](int item) -> const VT* {
@@ -2057,7 +2063,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
             bool ok = true;
             for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x)
             {
-                const int64_t row0 = tile * a.T;
+                const int64_t row0 = first_row(tile);
                 for (int item = 0; item < nitems; ++item)
                 {
                     if (*reinterpret_cast<volatile int*>(abort_flag)) { ok = false; break; }
@@ -2135,7 +2141,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
         };
         for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x)
         {
-            const int64_t row0 = tile * a.T;
+            const int64_t row0 = first_row(tile);
             // 9 warps put 3 on one scheduler: at most 168 registers/thread
             double w[R], vj[R];
             for (int item = 0; item < nitems; ++item)
