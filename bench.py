@@ -960,7 +960,8 @@ def run_dense(args):
     points uniform in the unit square (PCG64 seed 1), scale 0.02, every pair
     kept, diagonal shift --shift; FP32 row-major on the host.  256 probes,
     lanczos_degree 50, full reorthogonalisation.  The operator is the
-    tensor-core dense product (3-term TF32 split, FP32 accumulation)."""
+    tensor-core dense product (three BF16 parts, six products, FP32
+    accumulation)."""
     import torch
     import imate_b200 as ib
     from imate_b200 import _lib
@@ -980,7 +981,7 @@ def run_dense(args):
     torch.cuda.empty_cache()
 
     Aop = ib.Matrix(A32)
-    Aop.get_device_operator()  # upload + TF32 split, outside the timing
+    Aop.get_device_operator()  # upload + split, outside the timing
     eng = ib.EngineOptions(block_size=args.probes, rng="parity")
     kw = dict(method="slq", gpu=True, num_gpu_devices=1, return_info=True,
               min_num_samples=args.probes, max_num_samples=args.probes,
@@ -1006,22 +1007,21 @@ def run_dense(args):
     est = float(np.mean([float(tr) for tr, _ in outs]))
 
     # tensor roofline of the dense product: useful 2 n^2 b flops per call,
-    # issued as three TF32 products; TF32 runs at half the bf16 rate
+    # issued as six BF16 products
     nl, ms, _ = kstats["spmm"]
     per_call = ms / nl * 1e-3 if nl else float("nan")
     useful = 2.0 * n * n * args.probes / per_call / 1e12
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             bf16 = float(json.load(f)["bf16_tflops"])
-        src = "measured bf16 burst / 2"
+        src = "measured bf16 burst"
     except (OSError, KeyError, ValueError):
-        bf16, src = 1590.0, "fallback bf16 burst / 2"
-    tf32_peak = bf16 / 2.0
+        bf16, src = 1590.0, "fallback bf16 burst"
     # DRAM bytes per product from the committed ncu capture at n = 8192
     # (traffic there equals the algorithmic bytes: A parts once, probe parts
     # and Y once), scaled by the algorithmic bytes of this size
     t8 = ncu_traffic("dense") if args.probes == 256 else None
-    alg = lambda m: 8.0 * m * m + 12.0 * m * args.probes  # noqa: E731
+    alg = lambda m: 6.0 * m * m + 10.0 * m * args.probes  # noqa: E731
     traffic = t8 * alg(n) / alg(8192) if t8 else None
     line = {
         "workload_kind": "dense", "metric": "dense SLQ logdet probe*steps/s "
@@ -1038,10 +1038,10 @@ def run_dense(args):
                    "orthogonalize": args.orthogonalize, "rng": "parity",
                    "host_build_s": build_s,
                    "l2": "inputs larger than L2 (split matrix %.1f GB)"
-                         % (8.0 * n * n / 1e9)},
+                         % (6.0 * n * n / 1e9)},
         "roofline": {"bound": "tensor", "kernel": "k_dense_tc (+ probe "
-                     "split)", "achieved": 3.0 * useful, "peak": tf32_peak,
-                     "unit": "TFLOP/s", "frac": 3.0 * useful / tf32_peak,
+                     "split)", "achieved": 6.0 * useful, "peak": bf16,
+                     "unit": "TFLOP/s", "frac": 6.0 * useful / bf16,
                      "traffic": traffic, "peak_source": src,
                      "traffic_note": "DRAM bytes per product: ncu at n = "
                                      "8192 scaled by algorithmic bytes",

@@ -641,7 +641,7 @@ def _precision_info(J):
     # the same probes that the test suite holds this format to (None where
     # no such bar is tested)
     if getattr(op, "dense", False):
-        spmm = "dense, tensor cores (TF32 three-term products, FP32 sums)"
+        spmm = "dense, tensor cores (BF16 six-term products, FP32 sums)"
         bar = None
     elif getattr(op, "block_formats", None) and b in (128, 256):
         spmm = ("128-row blocks, tensor cores (FP16 three-product split of "

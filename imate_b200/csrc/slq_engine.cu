@@ -243,22 +243,20 @@ struct slq_op {
     const int32_t* t_gptr = nullptr;
     const int32_t* t_gcol = nullptr;
     const void* t_gval = nullptr;
-    // dense FP32 operator (tensor-core product): TF32 parts of A, [nrows][ldk],
-    // and of A^T, [ncols][ldk_t], K-major with zero-padded pitches; the
-    // probe-block parts scratch [256][ldx]; running totals of split products
+    // dense FP32 operator (tensor-core product): BF16 parts of A,
+    // [3][nrows][ldk], and of A^T, [3][ncols][ldk_t], K-major with zero-padded
+    // pitches; the probe-block parts scratch [3][256][ldx]; running totals of
+    // split products
     // (dense_ksplit of the SM count at creation); TMA maps of the A parts
     int dense = 0;
     float* d_acc = nullptr;
     int dense_sms = 0;
-    float* d_hi = nullptr;
-    float* d_lo = nullptr;
-    float* dt_hi = nullptr;
-    float* dt_lo = nullptr;
+    __nv_bfloat16* d_parts = nullptr;
+    __nv_bfloat16* dt_parts = nullptr;
+    __nv_bfloat16* xt_parts = nullptr;
     int64_t ldk = 0, ldk_t = 0, ldx = 0;
-    float* xt_hi = nullptr;
-    float* xt_lo = nullptr;
     int32_t* d_error = nullptr;
-    CUtensorMap map_hi, map_lo, map_t_hi, map_t_lo;
+    CUtensorMap map_parts, map_t_parts;
     // tensor-core block format (k_spmm_blk, FP32 operators) of A and of A^T:
     // 128-row blocks, first stage per block, union columns, row scales,
     // FP16 stage images
@@ -1110,7 +1108,7 @@ struct Launcher {
 // A launch that may overlap its predecessor's end (programmatic stream
 // serialization): only for kernels that call pdl_wait before they touch memory.
 template <typename... P, typename... A>
-slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                       A... args)
 {
     cudaLaunchAttribute attr{};
@@ -1118,7 +1116,7 @@ slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, int thre
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
@@ -1337,7 +1335,8 @@ slq_status make_xmaps(XMaps* m, const float* base, int64_t rows, int b, bool row
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
 struct DenseBufs {
-    float *hi, *lo, *t_hi, *t_lo, *x_hi, *x_lo, *acc;
+    __nv_bfloat16 *a, *t, *x;
+    float* acc;
     int32_t* error;
     int64_t ldk, ldk_t, ldx;
 };
@@ -1360,12 +1359,9 @@ void dense_layout(Carver& c, int64_t rows, int64_t cols, int need_transpose, int
     d->ldk = round_up(std::max<int64_t>(cols, 1), DT_BK);
     d->ldk_t = need_transpose ? round_up(std::max<int64_t>(rows, 1), DT_BK) : 0;
     d->ldx = std::max(d->ldk, d->ldk_t);
-    d->hi = c.take<float>(static_cast<size_t>(rows) * d->ldk);
-    d->lo = c.take<float>(static_cast<size_t>(rows) * d->ldk);
-    d->t_hi = need_transpose ? c.take<float>(static_cast<size_t>(cols) * d->ldk_t) : nullptr;
-    d->t_lo = need_transpose ? c.take<float>(static_cast<size_t>(cols) * d->ldk_t) : nullptr;
-    d->x_hi = c.take<float>(static_cast<size_t>(256) * d->ldx);
-    d->x_lo = c.take<float>(static_cast<size_t>(256) * d->ldx);
+    d->a = c.take<__nv_bfloat16>(static_cast<size_t>(3) * rows * d->ldk);
+    d->t = need_transpose ? c.take<__nv_bfloat16>(static_cast<size_t>(3) * cols * d->ldk_t) : nullptr;
+    d->x = c.take<__nv_bfloat16>(static_cast<size_t>(3) * 256 * d->ldx);
     // running totals of split products, for either direction
     int64_t acc_rows = dense_ksplit(rows, cols, sms) > 1 ? dense_ksplit(rows, cols, sms) * rows : 0;
     if (need_transpose && dense_ksplit(cols, rows, sms) > 1)
@@ -1374,10 +1370,10 @@ void dense_layout(Carver& c, int64_t rows, int64_t cols, int need_transpose, int
     d->error = c.take<int32_t>(1);
 }
 
-// K-major TF32-part tensor map: [outer][ld] FP32, box 32 x box_rows,
-// SWIZZLE_128B (128-byte rows)
-slq_status part_map(CUtensorMap* m, const float* base, int64_t ld, int64_t outer,
-                    int box_rows)
+// tensor map of K-major BF16 parts: [3][part_rows][ld], of which `outer` rows
+// of each part hold data, box 32 x box_rows x 3, SWIZZLE_64B (64-byte rows)
+slq_status part_map(CUtensorMap* m, const __nv_bfloat16* base, int64_t ld, int64_t part_rows,
+                    int64_t outer, int box_rows)
 {
     if (!g_encode_tiled)
     {
@@ -1388,13 +1384,15 @@ slq_status part_map(CUtensorMap* m, const float* base, int64_t ld, int64_t outer
             return fail(SLQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
         g_encode_tiled = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    cuuint64_t dims[2] = {static_cast<cuuint64_t>(ld), static_cast<cuuint64_t>(outer)};
-    cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * sizeof(float)};
-    cuuint32_t box[2] = {static_cast<cuuint32_t>(DT_BK), static_cast<cuuint32_t>(box_rows)};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = g_encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base),
-                                dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    const cuuint64_t pitch = static_cast<cuuint64_t>(ld) * sizeof(__nv_bfloat16);
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(ld), static_cast<cuuint64_t>(outer), 3};
+    cuuint64_t strides[2] = {pitch, pitch * static_cast<cuuint64_t>(part_rows)};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(DT_BK), static_cast<cuuint32_t>(box_rows), 3};
+    cuuint32_t es[3] = {1, 1, 1};
+    CUresult r = g_encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+                                const_cast<__nv_bfloat16*>(base), dims, strides, box, es,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return fail(SLQ_ERR_CUDA, "cuTensorMapEncodeTiled (dense) failed (" +
@@ -1402,11 +1400,16 @@ slq_status part_map(CUtensorMap* m, const float* base, int64_t ld, int64_t outer
     return SLQ_OK;
 }
 
-size_t dense_smem(int NB)
+size_t dense_stage(int NB) { return 3 * (128 + static_cast<size_t>(NB)) * DT_BK * 2; }
+
+// as many stages as fit (three of 72 KB at 256 probes)
+int dense_stages(int NB)
 {
-    const size_t stage = 2 * 128 * DT_BK * 4 + 2 * static_cast<size_t>(NB) * DT_BK * 4;
-    return 1023 + DT_STAGES * stage + 128 + 4 * 256 * sizeof(double);
+    return static_cast<int>(
+        std::min<size_t>(DT_MAX_STAGES, (232448 - 1023 - DT_TAIL) / dense_stage(NB)));
 }
+
+size_t dense_smem(int NB) { return 1023 + dense_stages(NB) * dense_stage(NB) + DT_TAIL; }
 
 // Y = A X (transpose: A^T X) on a dense operator, the SpMM epilogue fused;
 // at most 256 probes per GEMM launch.  *grid_out = the partial rows.
@@ -1415,12 +1418,11 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
                       const double* zc, const double* zs, int epi, double* partials,
                       int* grid_out, int32_t* error)
 {
-    if (transpose && !op->dt_hi)
+    if (transpose && !op->dt_parts)
         return fail(SLQ_ERR_BAD_ARG, "dense operator has no transpose");
     const int64_t M = transpose ? op->ncols : op->nrows;
     const int64_t K = transpose ? op->nrows : op->ncols;
-    const CUtensorMap& ahi = transpose ? op->map_t_hi : op->map_hi;
-    const CUtensorMap& alo = transpose ? op->map_t_lo : op->map_lo;
+    const CUtensorMap& a_parts = transpose ? op->map_t_parts : op->map_parts;
     const int64_t ntm = (M + 127) / 128;
     // split K when the row tiles leave most SMs idle (the same choice as the
     // scratch was sized for)
@@ -1429,10 +1431,10 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
     if (!attr)
     {
         SLQ_CK(cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(dense_smem(256))));
+                                    232448));
         attr = true;
     }
-    const double bytes = double(M) * K * 8.0 + double(K) * b * 4.0 + double(M) * b * 4.0;
+    const double bytes = double(M) * K * 6.0 + double(K) * b * 4.0 + double(M) * b * 4.0;
     ProfScope prof(SLQ_K_SPMM, bytes, L.st);
     // one grid for every chunk (the finalize reads the same partial rows for
     // all columns): the first chunk's, which has the most tiles; a CTA
@@ -1445,31 +1447,29 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
     {
         const int nb = std::min(256, b - p_off);
         // one probe tile per chunk: narrower tiles (more CTAs for small M)
-        // re-read the A tile from shared memory for less MMA work each and
-        // measured slower (n = 8192: 414 vs 369 us)
+        // would read A once per tile
         const int NB = static_cast<int>(round_up(nb, 16));
-        const int ntn = 1;
         if (grid_all == 0)
             grid_all = static_cast<int>(
-                std::max<int64_t>(1, std::min<int64_t>(ntm * ntn * ksplit, L.sms)));
+                std::max<int64_t>(1, std::min<int64_t>(ntm * ksplit, L.sms)));
         const int grid = grid_all;
-        dim3 tg(static_cast<unsigned>((K + 31) / 32), static_cast<unsigned>((nb + 31) / 32));
-        k_split_transpose<<<tg, dim3(32, 8), 0, L.st>>>(X, K, b, p_off, nb, op->ldx, op->xt_hi,
-                                                        op->xt_lo);
-        SLQ_LAUNCH_CK();
+        const int64_t pad = round_up(K, DT_BK);
+        dim3 tg(static_cast<unsigned>((pad + 63) / 64), static_cast<unsigned>((nb + 31) / 32));
+        SLQ_TRY(launch_pdl(L.st, k_dense_split_t, tg, dim3(32, 8), 0, X, K, int64_t(b),
+                           int64_t(p_off), int64_t(nb), pad, op->ldx, 256 * op->ldx,
+                           op->xt_parts));
         ++L.launches;
-        CUtensorMap xhi, xlo;
-        SLQ_TRY(part_map(&xhi, op->xt_hi, op->ldx, nb, NB));
-        SLQ_TRY(part_map(&xlo, op->xt_lo, op->ldx, nb, NB));
+        CUtensorMap x_parts;
+        SLQ_TRY(part_map(&x_parts, op->xt_parts, op->ldx, 256, nb, NB));
         DenseArgs d;
         d.M = M;
         d.K = K;
         d.nb = nb;
         d.NB = NB;
-        d.ntn = ntn;
+        d.stages = dense_stages(NB);
         d.b = b;
         d.p_off = p_off;
-        // running total and chunk accumulator: two power-of-two halves
+        // two chunk accumulators, a power of two columns each
         uint32_t cols = 32;
         while (cols < static_cast<uint32_t>(NB)) cols <<= 1;
         d.tmem_cols = 2 * cols;
@@ -1485,13 +1485,13 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
         d.error = error ? error : op->d_error;
         d.ksplit = ksplit;
         d.acc = op->d_acc;
-        k_dense_tc<<<grid, DT_THREADS, dense_smem(NB), L.st>>>(ahi, alo, xhi, xlo, d);
-        SLQ_LAUNCH_CK();
+        SLQ_TRY(launch_pdl(L.st, k_dense_tc, grid, DT_THREADS, dense_smem(NB), a_parts, x_parts, d));
         ++L.launches;
         if (ksplit > 1)
         {
-            k_dense_epi<<<epi_grid, 256, 0, L.st>>>(d);
-            SLQ_LAUNCH_CK();
+            int CP = 32;
+            while (CP < nb) CP <<= 1;
+            SLQ_TRY(launch_pdl(L.st, k_dense_epi, epi_grid, 256, 0, d, CP));
             ++L.launches;
         }
     }
@@ -2127,7 +2127,7 @@ slq_status make_plan(const slq_op* op, const slq_params* p, int q, RunPlan* r)
                     "eigenvalue shift across inquiries is not valid for Golub-Kahn runs");
     if (p->gram != 2 && op->nrows != op->ncols && (p->gram == 0 || op->affine))
         return fail(SLQ_ERR_BAD_ARG, "this run needs a square matrix");
-    if (p->gram && !(op->dense ? op->dt_hi != nullptr : op->t_ptr != nullptr))
+    if (p->gram && !(op->dense ? op->dt_parts != nullptr : op->t_ptr != nullptr))
         return fail(SLQ_ERR_BAD_ARG, "gram runs need an operator created with need_transpose");
     if (p->orthogonalize > p->lanczos_degree)
         return fail(SLQ_ERR_BAD_ARG, "orthogonalize must be at most lanczos_degree");
@@ -3301,7 +3301,7 @@ extern "C" slq_status slq_operator_dot(slq_op* op, int transpose, double t, cons
     if (x == y) return fail(SLQ_ERR_BAD_ARG, "operator_dot: x and y must not alias");
     if (!is_pow2(width) || width > ((op->dtype == SLQ_F64) ? 512 : 1024))
         return fail(SLQ_ERR_BAD_ARG, "operator_dot: width must be a power of two");
-    if (transpose && !(op->dense ? op->dt_hi != nullptr : op->t_ptr != nullptr))
+    if (transpose && !(op->dense ? op->dt_parts != nullptr : op->t_ptr != nullptr))
         return fail(SLQ_ERR_BAD_ARG, "operator_dot: operator has no transpose");
     Launcher L;
     L.st = static_cast<cudaStream_t>(stream);
@@ -3592,17 +3592,16 @@ extern "C" slq_status slq_dense_operator_create(const void* data, int64_t num_ro
     Carver c(workspace, workspace_bytes);
     DenseBufs d;
     dense_layout(c, num_rows, num_cols, need_transpose, sms, &d);
-    // zero padding, then the parts
-    SLQ_CK(cudaMemsetAsync(workspace, 0, c.off, st));
+    SLQ_CK(cudaMemsetAsync(d.error, 0, sizeof(int32_t), st));
     const float* A = static_cast<const float*>(data);
-    k_split_rows<<<sms * 8, 256, 0, st>>>(A, num_rows, num_cols, num_cols, d.ldk, d.hi, d.lo);
+    k_dense_split<<<sms * 8, 256, 0, st>>>(A, num_rows, num_cols, d.ldk, d.a);
     SLQ_LAUNCH_CK();
     if (need_transpose)
     {
-        dim3 tg(static_cast<unsigned>((num_rows + 31) / 32),
+        dim3 tg(static_cast<unsigned>((d.ldk_t + 63) / 64),
                 static_cast<unsigned>((num_cols + 31) / 32));
-        k_split_transpose<<<tg, dim3(32, 8), 0, st>>>(A, num_rows, num_cols, 0, num_cols,
-                                                      d.ldk_t, d.t_hi, d.t_lo);
+        k_dense_split_t<<<tg, dim3(32, 8), 0, st>>>(A, num_rows, num_cols, 0, num_cols, d.ldk_t,
+                                                    d.ldk_t, num_cols * d.ldk_t, d.t);
         SLQ_LAUNCH_CK();
     }
     slq_op* op = new slq_op();
@@ -3612,22 +3611,18 @@ extern "C" slq_status slq_dense_operator_create(const void* data, int64_t num_ro
     op->ncols = num_cols;
     op->nnz = num_rows * num_cols;
     op->dense = 1;
-    op->d_hi = d.hi;
-    op->d_lo = d.lo;
-    op->dt_hi = d.t_hi;
-    op->dt_lo = d.t_lo;
+    op->d_parts = d.a;
+    op->dt_parts = d.t;
+    op->xt_parts = d.x;
     op->ldk = d.ldk;
     op->ldk_t = d.ldk_t;
     op->ldx = d.ldx;
-    op->xt_hi = d.x_hi;
-    op->xt_lo = d.x_lo;
     op->d_acc = d.acc;
     op->dense_sms = sms;
     op->d_error = d.error;
-    slq_status s = part_map(&op->map_hi, d.hi, d.ldk, num_rows, 128);
-    if (s == SLQ_OK) s = part_map(&op->map_lo, d.lo, d.ldk, num_rows, 128);
-    if (s == SLQ_OK && need_transpose) s = part_map(&op->map_t_hi, d.t_hi, d.ldk_t, num_cols, 128);
-    if (s == SLQ_OK && need_transpose) s = part_map(&op->map_t_lo, d.t_lo, d.ldk_t, num_cols, 128);
+    slq_status s = part_map(&op->map_parts, d.a, d.ldk, num_rows, num_rows, 128);
+    if (s == SLQ_OK && need_transpose)
+        s = part_map(&op->map_t_parts, d.t, d.ldk_t, num_cols, num_cols, 128);
     if (s != SLQ_OK)
     {
         delete op;

@@ -21,6 +21,7 @@
 #ifndef SLQ_KERNELS_CUH_
 #define SLQ_KERNELS_CUH_
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <climits>
 #include <cstdint>
@@ -3307,102 +3308,127 @@ k_spmm_tc(const __grid_constant__ CUtensorMap xmap, const int32_t* __restrict__ 
 }
 
 // ===========================================================================
-// Dense operator product on the tensor cores (FP32 data, three TF32 terms).
+// Dense operator product on the tensor cores (FP32 data, six BF16 terms).
 //
-// Y[M][b] = A[M][K] X[K][b] for a dense row-major A.  A is split once into
-// TF32 parts, hi = rn_tf32(a), lo = rn_tf32(a - hi), stored K-major with a
-// row pitch ldk (a multiple of 32, zero-padded); each product splits and
-// transposes the probe block likewise (XT[p][k], k contiguous), at most 256
-// probes at a time.  A CTA computes 128-row tiles of Y (persistent over the
-// tiles): TMA loads 32-value K slices of A_hi, A_lo, XT_hi, XT_lo
-// (128-byte rows, SWIZZLE_128B) into a two-stage ring, one thread issues
-// per K step of 8 the three kind::tf32 MMAs A_hi XT_hi + A_hi XT_lo +
-// A_lo XT_hi into an FP32 accumulator in tensor memory (D[128][N], lane =
-// row, column = probe).  The tensor core's FP32 accumulation does not round
-// to nearest: its error is biased towards zero and grows with the number of
-// MMAs into one accumulator.  So each 128-value K chunk goes to a fresh
-// accumulator that four warps add into a running total (also in tensor
-// memory) with round-to-nearest FP32 adds, and then apply the SpMM epilogue
-// to it (thread t = row t of the tile).  Measured bias of Y (mean signed
-// error over mean |Y|, exponential-kernel matrices, n = 4096..16384):
-// 1.4e-6 with one accumulator per 512 values, 3.5e-7 per 128 at the same
-// speed for n >= 16384 (10 % slower at n = 4096), 1.7e-7 per 64 (25 %
-// slower at n = 4096).  The dropped lo*lo term and the rounding of the lo
-// parts leave ~2^-21 relative error per product.  Probe partial sums are
-// reduced across the tile's rows in a fixed order.
+// Y[M][b] = A[M][K] X[K][b] for a dense row-major A.  Each operand is split
+// into three BF16 parts, h = rn_bf16(v), m = rn_bf16(v - h) and l = v - h - m,
+// which hold all 24 bits and FP32's range.  The parts of A are made once,
+// [part][row][k] with a row pitch ldk (a multiple of 32, zero-padded); each
+// product splits and transposes the probe block likewise (XT[part][p][k], k
+// contiguous), at most 256 probes at a time.
+//
+// A CTA computes 128-row tiles of Y (persistent over the tiles): TMA loads
+// 32-value K slices of A's and XT's parts (64-byte rows, SWIZZLE_64B; one
+// copy brings all three parts) into a ring, one thread issues per K step of
+// 16 the six kind::f16 MMAs l h + m m + h l + m h + h m + h h (the terms
+// left out are below 2^-24) into an FP32 accumulator in tensor memory
+// (D[128][N], lane = row, column = probe).  The tensor core's FP32
+// accumulation does not round to nearest: its error is biased towards zero
+// and grows with the number of MMAs into one accumulator.  So each 64-value K
+// chunk goes to a fresh accumulator, two of them in turn, that eight warps
+// add into a running total in registers with round-to-nearest FP32 adds
+// while the next chunk's MMAs run; then they apply the SpMM epilogue (thread
+// = one row, half of the probes).
+//
+// What bounds it is the traffic from L2 into shared memory, mostly the probe
+// block that every tile reads again: six bytes a value against the eight of a
+// TF32 pair, whose three products take the tensor core as long as these six.
+// FP16 pairs would halve it, but drop what lies 2^-38 below the largest
+// element of a row or probe.  With 8192 x 8192 and 256 probes a product took
+// 258 us with TF32 pairs, one accumulator and two stages of four copies, and
+// takes 188 us (159 us of it this kernel, tensor pipe 81 % busy on 128 SMs);
+// the error against 64 bits is 2.3e-7 of |Y| (it was 4.5e-7).
 // ===========================================================================
 
-constexpr int DT_BK = 32;       // K values per stage (one 128-byte row)
-constexpr int DT_STAGES = 2;
-#ifndef SLQ_DT_CHUNK
-#define SLQ_DT_CHUNK 4
-#endif
-constexpr int DT_CHUNK = SLQ_DT_CHUNK;  // stages per accumulation chunk (128 K values)
-constexpr int DT_THREADS = 192; // warps 0-3 accumulate, 4 loads, 5 issues MMAs
-#ifndef SLQ_DT_PREFETCH
-#define SLQ_DT_PREFETCH 4
-#endif
-constexpr int DT_PREFETCH = SLQ_DT_PREFETCH;  // A stages prefetched into L2 ahead (0: none; 4 measured 3 % faster at n = 16384, no change at 4096-8192)
+constexpr int DT_BK = 32;       // K values per stage (one 64-byte row)
+constexpr int DT_MAX_STAGES = 8;
+constexpr int DT_CHUNK = 2;     // stages per accumulation chunk (64 K values)
+constexpr int DT_ACC_WARPS = 8; // warps 0-7 accumulate, 8 loads, 9 issues MMAs
+constexpr int DT_THREADS = (DT_ACC_WARPS + 2) * 32;
+constexpr int DT_PREFETCH = 4;  // A stages prefetched into L2 ahead (3 % faster than none at n = 16384, no change at 4096-8192)
+constexpr int DT_TAIL = 256 + 4 * 256 * 8;  // barriers, partial sums
+constexpr int DT_SEG = 2048;    // columns a warp takes of one row when A is split
 
-__device__ __forceinline__ void split_tf32_f(float x, float& hi, float& lo)
+// v = h + m + l, each BF16 (exact up to the underflow of l)
+__device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& h, __nv_bfloat16& m,
+                                           __nv_bfloat16& l)
 {
-    uint32_t h, l;
-    tc::split_tf32(x, h, l);
-    hi = __uint_as_float(h);
-    lo = __uint_as_float(l);
+    // a finite v stays finite: the largest BF16 value is a little below FP32's
+    constexpr float BF16_MAX = 3.3895313892515355e38f;
+    h = __float2bfloat16_rn(isfinite(v) ? fminf(fmaxf(v, -BF16_MAX), BF16_MAX) : v);
+    const float r = v - __bfloat162float(h);
+    m = __float2bfloat16_rn(r);
+    l = __float2bfloat16_rn(r - __bfloat162float(m));
 }
 
-// out[r * ldo + c] = parts of src[r * lds + c] for r < rows, c < cols
-__global__ void k_split_rows(const float* __restrict__ src, int64_t rows, int64_t cols,
-                             int64_t lds, int64_t ldo, float* __restrict__ hi,
-                             float* __restrict__ lo)
+// The parts of two adjacent values, to dst, dst + part and dst + 2 part
+__device__ __forceinline__ void split_store(float v0, float v1, __nv_bfloat16* dst, int64_t part)
 {
-    const int64_t total = rows * cols;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    __nv_bfloat162 h, m, l;
+    split_bf16(v0, h.x, m.x, l.x);
+    split_bf16(v1, h.y, m.y, l.y);
+    *reinterpret_cast<__nv_bfloat162*>(dst) = h;
+    *reinterpret_cast<__nv_bfloat162*>(dst + part) = m;
+    *reinterpret_cast<__nv_bfloat162*>(dst + 2 * part) = l;
+}
+
+// The parts of A, row pitch ldk (even), zero past the last column; warp =
+// DT_SEG columns of one row, lane = two of 64 adjacent ones
+__global__ void k_dense_split(const float* __restrict__ A, int64_t rows, int64_t cols,
+                              int64_t ldk, __nv_bfloat16* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t segs = (ldk + DT_SEG - 1) / DT_SEG;
+    for (int64_t u = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+         u < rows * segs; u += (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5)
     {
-        const int64_t r = i / cols, c = i % cols;
-        float h, l;
-        split_tf32_f(src[r * lds + c], h, l);
-        hi[r * ldo + c] = h;
-        lo[r * ldo + c] = l;
+        const int64_t r = u / segs;
+        const int64_t c0 = (u - r * segs) * DT_SEG;
+        const int64_t c1 = min(ldk, c0 + DT_SEG);
+#pragma unroll 4
+        for (int64_t c = c0 + 2 * lane; c < c1; c += 64)
+        {
+            const float v0 = c < cols ? A[r * cols + c] : 0.0f;
+            const float v1 = c + 1 < cols ? A[r * cols + c + 1] : 0.0f;
+            split_store(v0, v1, out + r * ldk + c, rows * ldk);
+        }
     }
 }
 
-// out[j * ldo + r] = parts of src[r * lds + col0 + j] for r < rows, j < ncols
-// (32 x 32 tiles through shared memory; block 32 x 8)
-__global__ void k_split_transpose(const float* __restrict__ src, int64_t rows, int64_t lds,
-                                  int64_t col0, int64_t ncols, int64_t ldo,
-                                  float* __restrict__ hi, float* __restrict__ lo)
+// out[j * ldo + r] = the parts (part elements apart) of src[r * lds + col0 +
+// j] for j < ncols, zero for rows <= r < pad (pad, ldo even).  64 x 32 tiles
+// through shared memory; block 32 x 8, lane = two adjacent r.
+__global__ void k_dense_split_t(const float* __restrict__ src, int64_t rows, int64_t lds,
+                                int64_t col0, int64_t ncols, int64_t pad, int64_t ldo,
+                                int64_t part, __nv_bfloat16* __restrict__ out)
 {
-    __shared__ float t[32][33];
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * 32;
+    __shared__ float t[64][33];
+    pdl_wait();
+    pdl_trigger();
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * 64;
     const int64_t c0 = static_cast<int64_t>(blockIdx.y) * 32;
-    for (int j = threadIdx.y; j < 32; j += 8)
+#pragma unroll
+    for (int j = threadIdx.y; j < 64; j += 8)
     {
         const int64_t r = r0 + j, c = c0 + threadIdx.x;
         t[j][threadIdx.x] = (r < rows && c < ncols) ? src[r * lds + col0 + c] : 0.0f;
     }
     __syncthreads();
+#pragma unroll
     for (int j = threadIdx.y; j < 32; j += 8)
     {
-        const int64_t c = c0 + j, r = r0 + threadIdx.x;
-        if (c < ncols && r < rows)
-        {
-            float h, l;
-            split_tf32_f(t[threadIdx.x][j], h, l);
-            hi[c * ldo + r] = h;
-            lo[c * ldo + r] = l;
-        }
+        const int64_t c = c0 + j, r = r0 + 2 * threadIdx.x;
+        if (c < ncols && r < pad)
+            split_store(t[2 * threadIdx.x][j], t[2 * threadIdx.x + 1][j], out + c * ldo + r, part);
     }
 }
 
 struct DenseArgs {
     int64_t M, K;        // rows of Y, inner dimension
-    int nb, NB, ntn;     // probes in this chunk; probes per tile (a multiple
-                         // of 16); probe tiles per row tile
+    int nb, NB;          // probes in this chunk; rounded up to a multiple of 16
+    int stages;          // ring stages
     int b, p_off;        // block width (row pitch of X, Y, Z) and chunk offset
-    uint32_t tmem_cols;  // power of two >= max(32, NB)
+    uint32_t tmem_cols;  // two accumulators: 2 x (power of two >= max(32, NB))
     const float* X;
     const double* sx;
     double shift;
@@ -3418,40 +3444,42 @@ struct DenseArgs {
 };
 
 __global__ void __launch_bounds__(DT_THREADS, 1)
-k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
-           const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ CUtensorMap x_lo,
+k_dense_tc(const __grid_constant__ CUtensorMap a_parts, const __grid_constant__ CUtensorMap x_parts,
            const DenseArgs d)
 {
     extern __shared__ __align__(1024) unsigned char smem_dense[];
-    // [stages][A_hi 16 KB | A_lo 16 KB | B_hi NB*128 | B_lo NB*128] at a
-    // 1024-aligned base, then barriers, tensor-memory address, reduction
-    const uint32_t a_bytes = 128 * DT_BK * 4;
-    const uint32_t b_bytes = static_cast<uint32_t>(d.NB) * DT_BK * 4;
-    const uint32_t stage_bytes = 2 * a_bytes + 2 * b_bytes;
+    // [stages][A h m l, 8 KB each | B h m l, NB * 64 each] at a 1024-aligned
+    // base, then barriers, tensor-memory address, reduction
+    const uint32_t a_bytes = 128 * DT_BK * 2;
+    const uint32_t b_bytes = static_cast<uint32_t>(d.NB) * DT_BK * 2;
+    const uint32_t stage_bytes = 3 * a_bytes + 3 * b_bytes;
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_dense) + 1023) & ~uintptr_t(1023));
-    unsigned char* tail = base + DT_STAGES * stage_bytes;
+    unsigned char* tail = base + d.stages * stage_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(tail);
-    uint64_t* empty = full + DT_STAGES;
-    uint64_t* chunk_full = empty + DT_STAGES;
-    uint64_t* chunk_empty = chunk_full + 1;
-    uint64_t* drain = chunk_empty + 1;
+    uint64_t* empty = full + DT_MAX_STAGES;
+    uint64_t* chunk_full = empty + DT_MAX_STAGES;  // [2]
+    uint64_t* chunk_empty = chunk_full + 2;        // [2]
+    uint64_t* drain = chunk_empty + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     int* abort_flag = reinterpret_cast<int*>(tmem_slot + 2);  // [2]
-    double* red = reinterpret_cast<double*>(tail + 128);     // [4][256]
+    double* red = reinterpret_cast<double*>(tail + 256);      // [4][256]
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
     if (tid == 0)
     {
-        for (int s = 0; s < DT_STAGES; ++s)
+        for (int s = 0; s < d.stages; ++s)
         {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(chunk_full, 1);
-        mbar_init(chunk_empty, 4);  // one arrival per accumulating warp
+        for (int c = 0; c < 2; ++c)
+        {
+            mbar_init(&chunk_full[c], 1);
+            mbar_init(&chunk_empty[c], DT_ACC_WARPS);  // one arrival per accumulating warp
+        }
         mbar_init(drain, 1);
         abort_flag[0] = 0;
         abort_flag[1] = 0;
@@ -3463,48 +3491,45 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
         tc::tmem_alloc(tmem_slot, d.tmem_cols);
         tc::tmem_relinquish();
     }
+    pdl_wait();
+    pdl_trigger();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    // running total in columns [0, NB), the chunk accumulator after it
-    const uint32_t d_chunk = tmem + d.tmem_cols / 2;
+    const uint32_t acc_stride = d.tmem_cols / 2;
 
-    // units: 128 rows x NB probes x one of ksplit K parts, the probe tiles of
-    // a row tile adjacent (they share the A stream through L2); part p of a
-    // tile takes the accumulation chunks [p nch / ksplit, (p + 1) nch / ksplit)
-    const int64_t ntiles = (d.M + 127) / 128 * d.ntn * d.ksplit;
+    // units: 128 rows x NB probes x one of ksplit K parts; part p of a tile
+    // takes the accumulation chunks [p nch / ksplit, (p + 1) nch / ksplit)
+    const int64_t ntiles = (d.M + 127) / 128 * d.ksplit;
     const int64_t nk = (d.K + DT_BK - 1) / DT_BK;
     const int64_t nch = (nk + DT_CHUNK - 1) / DT_CHUNK;  // chunks per tile
     auto k_range = [&](int64_t unit, int64_t& k0, int64_t& k1) {
         const int64_t part = unit % d.ksplit;
         k0 = part * nch / d.ksplit * DT_CHUNK;
-        k1 = std::min<int64_t>(nk, (part + 1) * nch / d.ksplit * DT_CHUNK);
+        k1 = min(nk, (part + 1) * nch / d.ksplit * DT_CHUNK);
     };
-    const uint32_t idesc = tc::idesc_tf32_m128(static_cast<uint32_t>(d.NB));
     auto give_up = [&]() {
         abort_flag[0] = 1;
         atomicExch(d.error, 1);
     };
 
-    if (warp == 4)
+    if (warp == DT_ACC_WARPS)
     {
         // producer: the A and probe-block parts of every stage of every tile
-        int64_t it = 0;
         if (lane == 0)
         {
+            int s = 0;
+            uint32_t ph = 0;
+            int64_t it = 0;
             bool ok = true;
             for (int64_t unit = blockIdx.x; unit < ntiles && ok; unit += gridDim.x)
             {
-                const int64_t tile = unit / d.ksplit;
-                const int row0 = static_cast<int>(tile / d.ntn * 128);
-                const int col0 = static_cast<int>(tile % d.ntn) * d.NB;
+                const int row0 = static_cast<int>(unit / d.ksplit * 128);
                 int64_t k0, k1;
                 k_range(unit, k0, k1);
                 for (int64_t k = k0; k < k1; ++k, ++it)
                 {
-                    const int s = static_cast<int>(it % DT_STAGES);
-                    const uint32_t ph = static_cast<uint32_t>((it / DT_STAGES) & 1);
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag))
                     {
                         give_up();
@@ -3514,52 +3539,42 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
                     unsigned char* st = base + static_cast<size_t>(s) * stage_bytes;
                     mbar_expect_tx(&full[s], stage_bytes);
                     const int kx = static_cast<int>(k * DT_BK);
-                    if (DT_PREFETCH > 0 && k + DT_PREFETCH < k1)
-                    {
-                        const int kp = static_cast<int>((k + DT_PREFETCH) * DT_BK);
-                        tc::tma_prefetch_2d(&a_hi, kp, row0);
-                        tc::tma_prefetch_2d(&a_lo, kp, row0);
-                    }
-                    tc::tma_load_2d(st, &a_hi, kx, row0, &full[s]);
-                    tc::tma_load_2d(st + a_bytes, &a_lo, kx, row0, &full[s]);
-                    tc::tma_load_2d(st + 2 * a_bytes, &x_hi, kx, col0, &full[s]);
-                    tc::tma_load_2d(st + 2 * a_bytes + b_bytes, &x_lo, kx, col0, &full[s]);
+                    if (k + DT_PREFETCH < k1)
+                        tc::tma_prefetch_3d(&a_parts, kx + DT_PREFETCH * DT_BK, row0, 0);
+                    tc::tma_load_3d(st, &a_parts, kx, row0, 0, &full[s]);
+                    tc::tma_load_3d(st + 3 * a_bytes, &x_parts, kx, 0, 0, &full[s]);
+                    if (++s == d.stages) { s = 0; ph ^= 1u; }
                 }
             }
             // the copies in flight land before the CTA leaves
-            for (int64_t k = it - DT_STAGES; k < it; ++k)
-            {
-                if (k < 0) continue;
-                mbar_wait(&full[k % DT_STAGES], static_cast<uint32_t>((k / DT_STAGES) & 1),
+            for (int64_t k = max(int64_t(0), it - d.stages); k < it; ++k)
+                mbar_wait(&full[k % d.stages], static_cast<uint32_t>((k / d.stages) & 1),
                           abort_flag + 1);
-            }
         }
         __syncwarp();
     }
-    else if (warp == 5)
+    else if (warp == DT_ACC_WARPS + 1)
     {
         // MMA issuer: one chunk accumulator per DT_CHUNK stages
         if (lane == 0)
         {
-            int64_t it = 0, cc = 0;
+            const uint32_t idesc = tc::idesc_bf16_m128(static_cast<uint32_t>(d.NB));
+            int s = 0;
+            uint32_t ph = 0;
+            int64_t cc = 0;
             bool ok = true;
             for (int64_t unit = blockIdx.x; unit < ntiles && ok; unit += gridDim.x)
             {
                 int64_t k0, k1;
                 k_range(unit, k0, k1);
-                for (int64_t k = k0; k < k1 && ok; ++k, ++it)
+                for (int64_t k = k0; k < k1; ++k)
                 {
                     const int64_t kc = (k - k0) % DT_CHUNK;
-                    if (kc == 0 && cc > 0 &&
-                        !mbar_wait(chunk_empty, static_cast<uint32_t>((cc - 1) & 1), abort_flag))
-                    {
-                        give_up();
-                        ok = false;
-                        break;
-                    }
-                    const int s = static_cast<int>(it % DT_STAGES);
-                    const uint32_t ph = static_cast<uint32_t>((it / DT_STAGES) & 1);
-                    if (!mbar_wait(&full[s], ph, abort_flag))
+                    const int buf = static_cast<int>(cc & 1);
+                    if ((kc == 0 && cc > 1 &&
+                         !mbar_wait(&chunk_empty[buf], static_cast<uint32_t>(((cc >> 1) - 1) & 1),
+                                    abort_flag)) ||
+                        !mbar_wait(&full[s], ph, abort_flag))
                     {
                         give_up();
                         ok = false;
@@ -3567,24 +3582,32 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
                     }
                     tc::fence_after_sync();
                     unsigned char* st = base + static_cast<size_t>(s) * stage_bytes;
-                    const uint64_t ah = tc::smem_desc_sw128(st);
-                    const uint64_t al = tc::smem_desc_sw128(st + a_bytes);
-                    const uint64_t bh = tc::smem_desc_sw128(st + 2 * a_bytes);
-                    const uint64_t bl = tc::smem_desc_sw128(st + 2 * a_bytes + b_bytes);
+                    const uint64_t ah = tc::smem_desc_sw64(st);
+                    const uint64_t am = tc::smem_desc_sw64(st + a_bytes);
+                    const uint64_t al = tc::smem_desc_sw64(st + 2 * a_bytes);
+                    unsigned char* bt = st + 3 * a_bytes;
+                    const uint64_t bh = tc::smem_desc_sw64(bt);
+                    const uint64_t bm = tc::smem_desc_sw64(bt + b_bytes);
+                    const uint64_t bl = tc::smem_desc_sw64(bt + 2 * b_bytes);
+                    const uint32_t dc = tmem + buf * acc_stride;
 #pragma unroll
-                    for (int kk = 0; kk < DT_BK / 8; ++kk)
+                    for (int kk = 0; kk < DT_BK / 16; ++kk)
                     {
-                        // K step kk: 8 TF32 values = 32 bytes further into each row
+                        // K step kk: 16 BF16 values = 32 bytes further into each row
                         const uint64_t o = static_cast<uint64_t>(kk * 32) >> 4;
                         const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
-                        tc::mma_tf32_ss(d_chunk, al + o, bh + o, idesc, acc);
-                        tc::mma_tf32_ss(d_chunk, ah + o, bl + o, idesc, 1u);
-                        tc::mma_tf32_ss(d_chunk, ah + o, bh + o, idesc, 1u);
+                        tc::mma_f16_ss(dc, al + o, bh + o, idesc, acc);
+                        tc::mma_f16_ss(dc, am + o, bm + o, idesc, 1u);
+                        tc::mma_f16_ss(dc, ah + o, bl + o, idesc, 1u);
+                        tc::mma_f16_ss(dc, am + o, bh + o, idesc, 1u);
+                        tc::mma_f16_ss(dc, ah + o, bm + o, idesc, 1u);
+                        tc::mma_f16_ss(dc, ah + o, bh + o, idesc, 1u);
                     }
                     tc::commit(&empty[s]);
+                    if (++s == d.stages) { s = 0; ph ^= 1u; }
                     if (kc == DT_CHUNK - 1 || k == k1 - 1)
                     {
-                        tc::commit(chunk_full);
+                        tc::commit(&chunk_full[buf]);
                         ++cc;
                     }
                 }
@@ -3597,87 +3620,99 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
     }
     else
     {
-        // warps 0-3: add each chunk into the running total (round to
-        // nearest), then the epilogue; thread tid owns tile row tid
+        // warps 0-7: add each chunk into the running total (round to
+        // nearest), then the epilogue; a thread owns one tile row and the
+        // first or second half of the probe columns, in groups of 16
+        const int rowlane = (warp & 3) * 32 + lane;
+        const int half = (d.NB / 16 + 1) / 2;  // groups of the first half
+        const int g0 = warp < 4 ? 0 : half;
+        const int ng = warp < 4 ? half : d.NB / 16 - half;
+        const uint32_t mine = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + g0 * 16;
         int64_t cc = 0;
         bool ok = true;
-        const uint32_t lanes = static_cast<uint32_t>(32 * warp) << 16;
         for (int64_t unit = blockIdx.x; unit < ntiles && ok; unit += gridDim.x)
         {
-            const int64_t tile = unit / d.ksplit;
             int64_t k0, k1;
             k_range(unit, k0, k1);
             const int64_t nch_u = (k1 - k0 + DT_CHUNK - 1) / DT_CHUNK;
+            float tot[8][16];
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) tot[g][j] = 0.0f;
             for (int64_t ch = 0; ch < nch_u; ++ch, ++cc)
             {
-                if (!__all_sync(FULL_MASK,
-                                mbar_wait(chunk_full, static_cast<uint32_t>(cc & 1), abort_flag)))
+                const int buf = static_cast<int>(cc & 1);
+                if (!__all_sync(FULL_MASK, mbar_wait(&chunk_full[buf],
+                                                     static_cast<uint32_t>((cc >> 1) & 1),
+                                                     abort_flag)))
                 {
                     if (lane == 0) give_up();
                     ok = false;
                     break;
                 }
                 tc::fence_after_sync();
-                for (int c0 = 0; c0 < d.NB; c0 += 16)
-                {
-                    uint32_t v[16], t[16];
-                    tc::ld_x16(d_chunk + lanes + c0, v);
-                    if (ch > 0) tc::ld_x16(tmem + lanes + c0, t);
-                    tc::wait_ld();
-                    if (ch > 0)
-                    {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            v[j] = __float_as_uint(__uint_as_float(t[j]) + __uint_as_float(v[j]));
+                for (int g = 0; g < 8; ++g)
+                    if (g < ng)
+                    {
+                        uint32_t v[16];
+                        tc::ld_x16(mine + buf * acc_stride + g * 16, v);
+                        tc::wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) tot[g][j] += __uint_as_float(v[j]);
                     }
-                    tc::st_x16(tmem + lanes + c0, v);
-                }
-                tc::wait_st();
                 tc::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(chunk_empty);
+                if (lane == 0) mbar_arrive(&chunk_empty[buf]);
             }
             if (!ok) break;
-            tc::fence_after_sync();
-            const int64_t row = tile / d.ntn * 128 + tid;
-            const int col0 = static_cast<int>(tile % d.ntn) * d.NB;
+            const int64_t row = unit / d.ksplit * 128 + rowlane;
             const bool live = row < d.M;
             if (d.ksplit > 1)
             {
                 // this part's running total; k_dense_epi adds the parts
-                float* dst = d.acc + ((unit % d.ksplit) * d.M + row) * d.NB + col0;
-                for (int c0 = 0; c0 < d.NB; c0 += 16)
+                if (live)
                 {
-                    uint32_t v[16];
-                    tc::ld_x16(tmem + lanes + c0, v);
-                    tc::wait_ld();
-                    if (live)
-                    {
+                    float4* dst = reinterpret_cast<float4*>(
+                        d.acc + ((unit % d.ksplit) * d.M + row) * d.NB + g0 * 16);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) dst[c0 + j] = __uint_as_float(v[j]);
-                    }
+                    for (int g = 0; g < 8; ++g)
+                        if (g < ng)
+                        {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                dst[g * 4 + j] = make_float4(tot[g][4 * j], tot[g][4 * j + 1],
+                                                             tot[g][4 * j + 2], tot[g][4 * j + 3]);
+                        }
                 }
-                tc::fence_before_sync();
                 continue;
             }
-            for (int c0 = 0; c0 < d.NB; c0 += 16)
+            // four columns at a time: the totals fill most of the registers
+#pragma unroll 1
+            for (int g4 = 0; g4 < 4 * ng; ++g4)
             {
-                uint32_t v[16];
-                tc::ld_x16(tmem + lanes + c0, v);
-                tc::wait_ld();
-                double add[16];
+                float v[4];
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
+                for (int k = 0; k < 32; ++k)
+                    if (k == g4)
+                    {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] = tot[k / 4][4 * (k & 3) + j];
+                    }
+                double add[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
                 {
                     add[j] = 0.0;
-                    const int q = col0 + c0 + j;
+                    const int q = g0 * 16 + g4 * 4 + j;
                     if (!live || q >= d.nb) continue;
                     const int p = d.p_off + q;
                     const int64_t o = row * d.b + p;
                     const double sxv = d.sx ? d.sx[p] : 1.0;
                     const float xv = (d.shift != 0.0 || d.epi == 1) ? d.X[o] : 0.0f;
                     const float zv = d.Z ? d.Z[o] : 0.0f;
-                    double y = static_cast<double>(__uint_as_float(v[j])) * sxv;
+                    double y = static_cast<double>(v[j]) * sxv;
                     if (d.shift != 0.0) y += d.shift * (sxv * static_cast<double>(xv));
                     if (d.Z) y -= (d.zc[p] * d.zs[p]) * static_cast<double>(zv);
                     const float yr = static_cast<float>(y);
@@ -3690,18 +3725,17 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
                 if (d.epi != 0)
                 {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
+                    for (int j = 0; j < 4; ++j)
                     {
                         double a = add[j];
 #pragma unroll
                         for (int off = 16; off > 0; off >>= 1)
                             a += __shfl_xor_sync(FULL_MASK, a, off);
-                        if (lane == 0 && col0 + c0 + j < d.nb)
-                            red[warp * 256 + col0 + c0 + j] += a;
+                        const int q = g0 * 16 + g4 * 4 + j;
+                        if (lane == 0 && q < d.nb) red[(warp & 3) * 256 + q] += a;
                     }
                 }
             }
-            tc::fence_before_sync();
         }
     }
 
@@ -3720,38 +3754,72 @@ k_dense_tc(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUt
 
 // The K parts of a split dense product: Y[r][p] from the ksplit running
 // totals (FP32 adds in part order), then the SpMM epilogue of k_dense_tc.
-// Block = 256 threads, thread q = probe column q of the chunk; block i takes
-// rows [i M / grid, (i + 1) M / grid) in order, so partials[i][p] is a
-// fixed-order sum over its rows.
+// Block = 256 threads = CP probe columns (a power of two, 32 .. 256, that
+// covers the chunk) x 256 / CP row lanes; block i takes rows [i M / grid,
+// (i + 1) M / grid), four rows of a lane at a time so that their loads
+// overlap.  partials[i][p] sums its rows in a fixed order.
 __global__ void __launch_bounds__(256)
-k_dense_epi(const DenseArgs d)
+k_dense_epi(const DenseArgs d, int CP)
 {
-    const int q = threadIdx.x;
-    if (q >= d.nb) return;
-    const int p = d.p_off + q;
-    const int64_t r0 = d.M * blockIdx.x / gridDim.x;
+    __shared__ double red[256];
+    constexpr int U = 4;
+    const int q = threadIdx.x % CP;
+    const int lanes = 256 / CP;
+    const int64_t r0 = d.M * blockIdx.x / gridDim.x + threadIdx.x / CP;
     const int64_t r1 = d.M * (blockIdx.x + 1) / gridDim.x;
-    const double sxv = d.sx ? d.sx[p] : 1.0;
-    const double zcs = d.Z ? d.zc[p] * d.zs[p] : 0.0;
+    const int p = d.p_off + q;
     double sum = 0.0;
-    for (int64_t row = r0; row < r1; ++row)
+    pdl_wait();
+    pdl_trigger();
+    if (q < d.nb)
     {
-        float t = d.acc[row * d.NB + q];
-        for (int k = 1; k < d.ksplit; ++k) t += d.acc[(k * d.M + row) * d.NB + q];
-        const int64_t o = row * d.b + p;
-        const float xv = (d.shift != 0.0 || d.epi == 1) ? d.X[o] : 0.0f;
-        const float zv = d.Z ? d.Z[o] : 0.0f;
-        double y = static_cast<double>(t) * sxv;
-        if (d.shift != 0.0) y += d.shift * (sxv * static_cast<double>(xv));
-        if (d.Z) y -= zcs * static_cast<double>(zv);
-        const float yr = static_cast<float>(y);
-        d.Y[o] = yr;
-        const double ys = static_cast<double>(yr);
-        if (d.epi == 1) sum += (sxv * static_cast<double>(xv)) * ys;
-        else if (d.epi == 2) sum += ys * ys;
-        else if (d.epi == 3) sum += (d.zs[p] * static_cast<double>(zv)) * ys;
+        const double sxv = d.sx ? d.sx[p] : 1.0;
+        const double zcs = d.Z ? d.zc[p] * d.zs[p] : 0.0;
+        const double zsv = d.epi == 3 ? d.zs[p] : 0.0;
+        const bool need_x = d.shift != 0.0 || d.epi == 1;
+        for (int64_t row0 = r0; row0 < r1; row0 += U * lanes)
+        {
+            float t[U], xv[U], zv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const int64_t row = row0 + u * lanes;
+                t[u] = xv[u] = zv[u] = 0.0f;
+                if (row >= r1) continue;
+                t[u] = d.acc[row * d.NB + q];
+                if (need_x) xv[u] = d.X[row * d.b + p];
+                if (d.Z) zv[u] = d.Z[row * d.b + p];
+            }
+            for (int k = 1; k < d.ksplit; ++k)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    const int64_t row = row0 + u * lanes;
+                    if (row < r1) t[u] += d.acc[(k * d.M + row) * d.NB + q];
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const int64_t row = row0 + u * lanes;
+                if (row >= r1) continue;
+                double y = static_cast<double>(t[u]) * sxv;
+                if (d.shift != 0.0) y += d.shift * (sxv * static_cast<double>(xv[u]));
+                if (d.Z) y -= zcs * static_cast<double>(zv[u]);
+                const float yr = static_cast<float>(y);
+                d.Y[row * d.b + p] = yr;
+                const double ys = static_cast<double>(yr);
+                if (d.epi == 1) sum += (sxv * static_cast<double>(xv[u])) * ys;
+                else if (d.epi == 2) sum += ys * ys;
+                else if (d.epi == 3) sum += (zsv * static_cast<double>(zv[u])) * ys;
+            }
+        }
     }
-    if (d.epi != 0) d.partials[static_cast<int64_t>(blockIdx.x) * d.b + p] = sum;
+    if (d.epi == 0) return;
+    red[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x >= d.nb || threadIdx.x >= CP) return;
+    for (int k = 1; k < lanes; ++k) sum += red[k * CP + q];
+    d.partials[static_cast<int64_t>(blockIdx.x) * d.b + p] = sum;
 }
 
 // ===========================================================================

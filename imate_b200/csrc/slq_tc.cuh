@@ -212,37 +212,42 @@ __host__ __device__ constexpr uint32_t idesc_tf32_m128(uint32_t n)
     return 0x00000910u | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-// Shared-memory descriptor of a K-major tile written by a SWIZZLE_128B TMA
-// load (rows of 128 bytes = 32 TF32 values, 8-row atoms of 1024 bytes):
-// stride byte offset 1024, leading byte offset unused (1), version 1, layout
-// type SWIZZLE_128B (2 in bits 61-63).  The tile must start on a 1024-byte
-// boundary; a K step of 8 values inside the atom advances the start by 32
-// bytes.
-__device__ __forceinline__ uint64_t smem_desc_sw128(const void* p)
+// The same with BF16 operands (kind::f16; type 1 in bits 7-9 and 10-12).
+__host__ __device__ constexpr uint32_t idesc_bf16_m128(uint32_t n)
 {
-    const uint64_t start = (smem_addr(p) >> 4) & 0x3FFFu;
-    return start | (uint64_t(1) << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) |
-           (uint64_t(2) << 61);
+    return 0x00000490u | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-// 2-D tiled TMA load of box (x, y) .. into shared memory, completing on bar.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
+// Shared-memory descriptor of a K-major tile written by a SWIZZLE_64B TMA
+// load (rows of 64 bytes = 32 BF16 values, 8-row atoms of 512 bytes): stride
+// byte offset 512, leading byte offset unused (1), version 1, layout type
+// SWIZZLE_64B (4 in bits 61-63).  The tile must start on a 512-byte boundary;
+// a K step of 16 values inside the atom advances the start by 32 bytes.
+__device__ __forceinline__ uint64_t smem_desc_sw64(const void* p)
+{
+    const uint64_t start = (smem_addr(p) >> 4) & 0x3FFFu;
+    return start | (uint64_t(1) << 16) | (uint64_t(512 >> 4) << 32) | (uint64_t(1) << 46) |
+           (uint64_t(4) << 61);
+}
+
+// 3-D tiled TMA load of box (x, y, z) .. into shared memory, completing on bar.
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             uint64_t* bar)
 {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y),
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z),
           "r"(smem_addr(bar))
         : "memory");
 }
 
-// L2 prefetch of one box of a 2-D tiled tensor map (no completion to wait
-// on; coordinates as tma_load_2d)
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y)
+// L2 prefetch of one box of a 3-D tiled tensor map (no completion to wait
+// on; coordinates as tma_load_3d)
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z)
 {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 

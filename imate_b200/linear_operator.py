@@ -599,7 +599,7 @@ class _DeviceOperator:
     @classmethod
     def from_dense(cls, A, affine=False, need_transpose=False):
         """Dense float32 operator over a host array A (row-major copy on the
-        device; ``slq_dense_operator_create``: TF32 parts of A, and of A^T
+        device; ``slq_dense_operator_create``: BF16 parts of A, and of A^T
         with ``need_transpose``, for the tensor-core product)."""
         import torch
         self = cls(None, affine, need_transpose)
