@@ -1931,8 +1931,9 @@ slq_status op_spmm(Launcher& L, const slq_op* op, int transpose, int b, const VT
                          partials, grid_out, maps, error);
 }
 
-// TMA-streamed pass (k_stream): MODE 0 = update + inner products,
-// MODE 1 = (update +) reorthogonalisation update + norm.
+// A pass over the Krylov vectors.  MODE 0 = update + inner products
+// (k_stream), MODE 1 = reorthogonalisation update + norm (k_reorth), without
+// basis vectors the three-term update + norm (k_three_term).
 template <typename VT, int MODE>
 slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int do_update,
                        const VT* Vj, const double* sj, const double* aj, const VT* Vm,
@@ -1949,22 +1950,25 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     constexpr size_t TILE = static_cast<size_t>(R) * STREAM_CONSUMERS * sizeof(VT);
     const int PT = std::min(b, STREAM_CONSUMERS);
     const int T = R * (STREAM_CONSUMERS / PT);
-    const size_t fixed = STREAM_BARRIER_BYTES + STREAM_CONSUMERS * sizeof(double);
-    const size_t extra = (MODE == 0) ? static_cast<size_t>(J) * STREAM_CONSUMERS * 8
-                                     : static_cast<size_t>(J) * PT * 8;
-    if (fixed + extra + 2 * TILE > SMEM_MAX)
-        return fail(SLQ_ERR_BAD_ARG, "stream pass: too many basis vectors per launch");
-    const int S = static_cast<int>(std::min<size_t>(STREAM_RING_BYTES / TILE,
-                                                    (SMEM_MAX - fixed - extra) / TILE));
-    const size_t smem = fixed + static_cast<size_t>(S) * TILE + extra;
-    auto kernel = (MODE == 1 && J == 0) ? k_stream<VT, MODE, R, false>
-                                        : k_stream<VT, MODE, R, MODE == 1>;
-    static bool attr[2] = {false, false};
-    if (!attr[J == 0])
+    int S = 0;
+    size_t smem = 0;
+    if constexpr (MODE == 0)
     {
-        SLQ_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(SMEM_MAX)));
-        attr[J == 0] = true;
+        const size_t fixed = STREAM_BARRIER_BYTES + STREAM_CONSUMERS * sizeof(double);
+        const size_t extra = static_cast<size_t>(J) * STREAM_CONSUMERS * 8;
+        if (fixed + extra + 2 * TILE > SMEM_MAX)
+            return fail(SLQ_ERR_BAD_ARG, "stream pass: too many basis vectors per launch");
+        S = static_cast<int>(std::min<size_t>(STREAM_RING_BYTES / TILE,
+                                              (SMEM_MAX - fixed - extra) / TILE));
+        smem = fixed + static_cast<size_t>(S) * TILE + extra;
+        static bool attr = false;
+        if (!attr)
+        {
+            SLQ_CK(cudaFuncSetAttribute(k_stream<VT, R>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(SMEM_MAX)));
+            attr = true;
+        }
     }
     StreamArgs<VT> a;
     a.n = n;
@@ -1998,8 +2002,18 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     a.x16exp = x16exp;
     if (g_fail_stream_waits.load() > 0 && g_fail_stream_waits.fetch_sub(1) > 0)
         a.fail_first_wait = 1;
-    const int gy = b / PT;
-    const int gx = std::max(1, L.sms / gy);
+    // one CTA per SM; the three-term update takes all probes of a row together.
+    // No more CTAs than 16-byte pieces for all threads: every CTA is a row of
+    // partial sums to add.
+    const bool plain = MODE == 1 && J == 0;
+    const int gy = plain ? 1 : b / PT;
+    int gx = plain ? THREE_TERM_CTAS * L.sms : std::max(1, L.sms / gy);
+    if constexpr (MODE == 1)
+    {
+        const int64_t step = (plain ? THREE_TERM_THREADS : REORTH_THREADS) * (16 / sizeof(VT));
+        gx = static_cast<int>(
+            std::max<int64_t>(1, std::min<int64_t>(gx, (n * b / gy + step - 1) / step)));
+    }
     const double vb = double(n) * b * sizeof(VT);
     const int npre = 1 + (do_update ? (Vm ? 2 : 1) : 0);
     const int skip = (MODE == 0 && do_update) ? (Vm ? 2 : 1) : 0;
@@ -2007,7 +2021,14 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     // the split parts: 2 x 2 bytes per element, one float vector's bytes
     const int writes = ((MODE == 1 || do_update) ? 1 : 0) + (x16 ? 1 : 0);
     ProfScope prof(MODE == 0 ? SLQ_K_DOTS : SLQ_K_REORTH, vb * (reads + writes), L.st);
-    SLQ_TRY(launch_pdl(L.st, kernel, dim3(gx, gy), STREAM_THREADS, smem, a));
+    if constexpr (MODE == 0)
+        SLQ_TRY(launch_pdl(L.st, k_stream<VT, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
+    else if (J > 0 && b * sizeof(VT) >= 16)
+        SLQ_TRY(launch_pdl(L.st, k_reorth<VT, false>, dim3(gx, gy), REORTH_THREADS, 0, a));
+    else if (J > 0)
+        SLQ_TRY(launch_pdl(L.st, k_reorth<VT, true>, dim3(gx, gy), REORTH_THREADS, 0, a));
+    else
+        SLQ_TRY(launch_pdl(L.st, k_three_term<VT>, gx, THREE_TERM_THREADS, 0, a));
     ++L.launches;
     *grid_out = gx;
     return SLQ_OK;

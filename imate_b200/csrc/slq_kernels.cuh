@@ -1940,6 +1940,23 @@ __device__ __forceinline__ void x16_store(__half* x16, int64_t row, int b, int p
     x16[row * 2 * b + b + p] = l;
 }
 
+// the same for four adjacent probes, p and b multiples of 4
+__device__ __forceinline__ void x16_store(__half* x16, int64_t row, int b, int p,
+                                          const float (&v)[4])
+{
+    const __half2 h0 = __floats2half2_rn(v[0], v[1]);
+    const __half2 h1 = __floats2half2_rn(v[2], v[3]);
+    const float2 f0 = __half22float2(h0);
+    const float2 f1 = __half22float2(h1);
+    const __half2 l0 = __floats2half2_rn(v[0] - f0.x, v[1] - f0.y);
+    const __half2 l1 = __floats2half2_rn(v[2] - f1.x, v[3] - f1.y);
+    __half* dst = x16 + row * 2 * b + p;
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0),
+                                                *reinterpret_cast<const uint32_t*>(&h1));
+    *reinterpret_cast<uint2*>(dst + b) = make_uint2(*reinterpret_cast<const uint32_t*>(&l0),
+                                                    *reinterpret_cast<const uint32_t*>(&l1));
+}
+
 template <typename VT>
 struct StreamArgs {
     int64_t n;            // rows
@@ -1979,15 +1996,12 @@ struct StreamArgs {
     int32_t* x16exp;
 };
 
-// MODE 0: dots, MODE 1: reorth.  R = rows per consumer thread per tile.
-// PAIR: MODE 1 takes two basis tiles per turn; without basis vectors (J = 0,
-// the plain three-term update) the code for it only costs (524,175 x 256 FP32:
-// 346 us without it, 372 with).
-template <typename VT, int MODE, int R, bool PAIR>
+// The dots pass.  R = rows per consumer thread per tile.
+template <typename VT, int R>
 __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<VT> a)
 {
     // shared memory: barriers | norm partials (256 doubles) | S stages of
-    // R x 256 values | dots: acc[J][256] doubles, reorth: coef[J][PT]
+    // R x 256 values | acc[J][256] doubles
     extern __shared__ __align__(128) unsigned char smem_stream[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_stream);
     uint64_t* empty = full + STREAM_MAX_STAGES;
@@ -2011,7 +2025,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
     const bool upd = a.do_update != 0;
     const int npre = 1 + (upd ? (a.Vm ? 2 : 1) : 0);
     // dots: basis vectors v_j, v_{j-1} are served from the update registers
-    const int skip = (MODE == 0 && upd) ? (a.Vm ? 2 : 1) : 0;
+    const int skip = upd ? (a.Vm ? 2 : 1) : 0;
     const int nbasis = (J > skip) ? J - skip : 0;
     const int nitems = npre + nbasis;
 
@@ -2026,24 +2040,12 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
         abort_flag[1] = 0;  // stays 0: bounded waits on the way out
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (MODE == 0)
-        for (int i = tid; i < J * STREAM_CONSUMERS; i += STREAM_THREADS) extra[i] = 0.0;
+    for (int i = tid; i < J * STREAM_CONSUMERS; i += STREAM_THREADS) extra[i] = 0.0;
     pdl_wait();
     pdl_trigger();
-    if (MODE == 1)
-    {
-        for (int i = tid; i < J * PT; i += STREAM_THREADS)
-            extra[i] = static_cast<double>(a.coef[static_cast<int64_t>(i / PT) * b + p0 + i % PT]);
-    }
     __syncthreads();
 
     const int64_t ntiles = a.n / a.T;
-    // MODE 1 walks the tiles backwards: it starts on what the pass (or product)
-    // before it read and wrote last, which is still in L2, and ends where the
-    // next product starts
-    auto first_row = [&](int64_t tile) {
-        return (MODE == 1 ? ntiles - 1 - tile : tile) * a.T;
-    };
     const bool contiguous = (PT == b);
     constexpr uint32_t tile_bytes = TILE * sizeof(VT);
     auto item_ptr = [&](int item) -> const VT* {
@@ -2064,7 +2066,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
             bool ok = true;
             for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x)
             {
-                const int64_t row0 = first_row(tile);
+                const int64_t row0 = tile * a.T;
                 for (int item = 0; item < nitems; ++item)
                 {
                     if (*reinterpret_cast<volatile int*>(abort_flag)) { ok = false; break; }
@@ -2118,23 +2120,6 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
         }
         double nacc = 0.0;
         bool ok = true;
-        // the split probe block (MODE 1 with x16): this probe's 2^e_p from
-        // the reduced |w|^2 partials of the dots pass (a fixed order)
-        bool x16_on = false;
-        float x16_scale = 1.0f;
-        if constexpr (MODE == 1 && sizeof(VT) == 4)
-        {
-            if (a.x16 && a.wn2_in)
-            {
-                double n2 = 0.0;
-                for (int g = 0; g < a.wn2_grid; ++g)
-                    n2 += a.wn2_in[static_cast<int64_t>(g) * b + p0 + pl];
-                const int e = (n2 > 0.0 && isfinite(n2)) ? x16_exp(1.0 / sqrt(n2)) : 0;
-                x16_scale = ldexpf(1.0f, e);
-                x16_on = true;
-                if (roff == 0 && blockIdx.x == 0) a.x16exp[p0 + pl] = e;
-            }
-        }
         const int lane = tid & 31;
         auto release = [&](int st) {
             __syncwarp();
@@ -2142,13 +2127,13 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
         };
         for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x)
         {
-            const int64_t row0 = first_row(tile);
+            const int64_t row0 = tile * a.T;
             // 9 warps put 3 on one scheduler: at most 168 registers/thread
             double w[R], vj[R];
             for (int item = 0; item < nitems; ++item)
             {
                 if (*reinterpret_cast<volatile int*>(abort_flag)) { ok = false; break; }
-                if (MODE == 0 && item >= npre && item + 1 < nitems)
+                if (item >= npre && item + 1 < nitems)
                 {
                     // dots: two basis tiles per turn, four FMA chains each, so
                     // the two load -> convert -> FMA -> add-tree chains overlap
@@ -2188,47 +2173,11 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                     ++item;
                     continue;
                 }
-                if (MODE == 1 && PAIR && item >= npre && item + 1 < nitems)
-                {
-                    // reorth: two basis tiles per turn as well, so that their
-                    // loads and conversions overlap (262,144 x 256 FP32,
-                    // J = 25: 1,252 -> 1,197 us)
-                    const int ib = skip + (item - npre);
-                    const double c0 = extra[ib * PT + pl];
-                    const double c1 = extra[(ib + 1) * PT + pl];
-                    int s1 = s + 1;
-                    uint32_t ph1 = phase;
-                    if (s1 == a.S) { s1 = 0; ph1 ^= 1; }
-                    if (!mbar_wait(&full[s], phase, abort_flag) ||
-                        !mbar_wait(&full[s1], ph1, abort_flag))
-                    {
-                        *abort_flag = 1;
-                        atomicExch(a.error, 1);
-                        ok = false;
-                        break;
-                    }
-                    const VT* t0 = stages + static_cast<size_t>(s) * TILE;
-                    const VT* t1 = stages + static_cast<size_t>(s1) * TILE;
-#pragma unroll
-                    for (int k = 0; k < R; ++k)
-                    {
-                        const int e = (roff + k * RSTEP) * PT + pl;
-                        w[k] -= c0 * static_cast<double>(t0[e]);
-                        w[k] -= c1 * static_cast<double>(t1[e]);
-                    }
-                    release(s);
-                    release(s1);
-                    s = s1 + 1;
-                    phase = ph1;
-                    if (s == a.S) { s = 0; phase ^= 1; }
-                    ++item;
-                    continue;
-                }
                 // dots: fetch this thread's running sum before the wait so the
                 // shared-memory latency overlaps it
                 const int ib = skip + (item - npre);
                 double prev = 0.0;
-                if (MODE == 0 && item >= npre) prev = extra[ib * STREAM_CONSUMERS + tid];
+                if (item >= npre) prev = extra[ib * STREAM_CONSUMERS + tid];
                 // the test hook makes the first wait of the launch run out
                 // (the simulated timeout takes the abort path below)
                 const bool first = tile == blockIdx.x && item == 0;
@@ -2263,28 +2212,17 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                 }
                 else
                 {
-                    const int i = ib;
-                    if (MODE == 0)
-                    {
-                        // eight independent FMA chains: the pass is bound by
-                        // the latency of this reduction (two warps per
-                        // scheduler), not by FP64 throughput
-                        double l[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                    // eight independent FMA chains: the pass is bound by the
+                    // latency of this reduction (two warps per scheduler),
+                    // not by FP64 throughput
+                    double l[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                        for (int k = 0; k < R; ++k)
-                            l[k & 7] += static_cast<double>(st[(roff + k * RSTEP) * PT + pl]) * w[k];
-                        extra[i * STREAM_CONSUMERS + tid] =
-                            prev + (((l[0] + l[1]) + (l[2] + l[3])) + ((l[4] + l[5]) + (l[6] + l[7])));
-                    }
-                    else
-                    {
-                        const double c = extra[i * PT + pl];
-#pragma unroll
-                        for (int k = 0; k < R; ++k)
-                            w[k] -= c * static_cast<double>(st[(roff + k * RSTEP) * PT + pl]);
-                    }
+                    for (int k = 0; k < R; ++k)
+                        l[k & 7] += static_cast<double>(st[(roff + k * RSTEP) * PT + pl]) * w[k];
+                    extra[ib * STREAM_CONSUMERS + tid] =
+                        prev + (((l[0] + l[1]) + (l[2] + l[3])) + ((l[4] + l[5]) + (l[6] + l[7])));
                 }
-                if (MODE == 0 && upd && item == npre - 1)
+                if (upd && item == npre - 1)
                 {
                     // updated w: round to storage, store, and serve the
                     // products with v_j (registers) and v_{j-1} (still in
@@ -2306,20 +2244,6 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                 }
                 release(s);
                 if (++s == a.S) { s = 0; phase ^= 1; }
-            }
-            if (MODE == 1 && ok)
-            {
-#pragma unroll
-                for (int k = 0; k < R; ++k)
-                {
-                    const VT wr = static_cast<VT>(w[k]);
-                    const double d = static_cast<double>(wr);
-                    nacc += d * d;
-                    const int64_t row = row0 + roff + k * RSTEP;
-                    a.Wout[row * b + p0 + pl] = wr;
-                    if (x16_on)
-                        x16_store(a.x16, row, b, p0 + pl, static_cast<float>(wr) * x16_scale);
-                }
             }
         }
 
@@ -2343,31 +2267,18 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                         y = static_cast<double>(a.Vm[o]);
                         wv -= cm * y;
                     }
-                    if (MODE == 0)
-                    {
-                        const VT wr = static_cast<VT>(wv);
-                        wv = static_cast<double>(wr);
-                        a.Wout[o] = wr;
-                        nacc += wv * wv;
-                        if (J > 0) extra[tid] += x * wv;
-                        if (a.Vm && J > 1) extra[STREAM_CONSUMERS + tid] += y * wv;
-                    }
+                    const VT wr = static_cast<VT>(wv);
+                    wv = static_cast<double>(wr);
+                    a.Wout[o] = wr;
+                    nacc += wv * wv;
+                    if (J > 0) extra[tid] += x * wv;
+                    if (a.Vm && J > 1) extra[STREAM_CONSUMERS + tid] += y * wv;
                 }
 #pragma unroll 4
                 for (int i = skip; i < J; ++i)
                 {
                     const VT* vp = a.basis + static_cast<int64_t>(ring_slot(a.last - i, a.bs)) * a.slot_elems;
-                    const double v = static_cast<double>(vp[o]);
-                    if (MODE == 0) extra[i * STREAM_CONSUMERS + tid] += v * wv;
-                    else wv -= extra[i * PT + pl] * v;
-                }
-                if (MODE == 1)
-                {
-                    const VT wr = static_cast<VT>(wv);
-                    const double d = static_cast<double>(wr);
-                    nacc += d * d;
-                    a.Wout[o] = wr;
-                    if (x16_on) x16_store(a.x16, r, b, p0 + pl, static_cast<float>(wr) * x16_scale);
+                    extra[i * STREAM_CONSUMERS + tid] += static_cast<double>(vp[o]) * wv;
                 }
             }
         }
@@ -2376,27 +2287,15 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
     __syncthreads();
 
     if (producer) return;
-    if (MODE == 0)
+    for (int idx = tid; idx < J * PT; idx += STREAM_CONSUMERS)
     {
-        for (int idx = tid; idx < J * PT; idx += STREAM_CONSUMERS)
-        {
-            const int i = idx / PT;
-            const int q = idx % PT;
-            double sum = 0.0;
-            for (int r = 0; r < RSTEP; ++r) sum += extra[i * STREAM_CONSUMERS + r * PT + q];
-            a.partials[(static_cast<int64_t>(blockIdx.x) * J + i) * b + p0 + q] = sum;
-        }
+        const int i = idx / PT;
+        const int q = idx % PT;
+        double sum = 0.0;
+        for (int r = 0; r < RSTEP; ++r) sum += extra[i * STREAM_CONSUMERS + r * PT + q];
+        a.partials[(static_cast<int64_t>(blockIdx.x) * J + i) * b + p0 + q] = sum;
     }
-    else if (a.want_norm)
-    {
-        for (int q = tid; q < PT; q += STREAM_CONSUMERS)
-        {
-            double sum = 0.0;
-            for (int r = 0; r < RSTEP; ++r) sum += red[r * PT + q];
-            a.partials[static_cast<int64_t>(blockIdx.x) * b + p0 + q] = sum;
-        }
-    }
-    if (MODE == 0 && a.wn2_out)
+    if (a.wn2_out)
     {
         for (int q = tid; q < PT; q += STREAM_CONSUMERS)
         {
@@ -2407,6 +2306,353 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
     }
 }
 
+
+// ===========================================================================
+// The update passes: plain 16-byte loads into registers.
+//
+// w is read once, the vectors stream past it once, nothing is shared between
+// threads but the norm: there is nothing to stage.  The TMA ring these passes
+// had cost its consumers a wait, a shared load and a hand-back per tile, and
+// whole 16 KB tiles left a last wave; plain loads keep as many bytes in flight
+// from registers and read HBM at 7.4 instead of 7.0 TB/s.
+//
+// A thread takes 16 bytes (VEC probes of a row) at a time; the pieces of
+// THREADS x 16 bytes go round the CTAs, from the last row back: the pass
+// starts on what the one before it read and wrote last, which is still in L2,
+// and ends where the next product starts.
+// ===========================================================================
+
+// 16 bytes that pass through once; kept behind pdl_wait by the volatile
+__device__ __forceinline__ void load_once(const float* p, float (&v)[4])
+{
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "l"(p));
+}
+
+__device__ __forceinline__ void load_once(const double* p, double (&v)[2])
+{
+    asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];"
+                 : "=d"(v[0]), "=d"(v[1])
+                 : "l"(p));
+}
+
+__device__ __forceinline__ void load_vec(const float* p, float (&v)[4])
+{
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+
+__device__ __forceinline__ void load_vec(const double* p, double (&v)[2])
+{
+    const double2 x = *reinterpret_cast<const double2*>(p);
+    v[0] = x.x; v[1] = x.y;
+}
+
+__device__ __forceinline__ void store_vec(float* p, const float (&v)[4])
+{
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ void store_vec(double* p, const double (&v)[2])
+{
+    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
+
+// Norm partials of a CTA: nacc[i] of thread t belongs to value t VEC + i of a
+// piece, whose probe is that modulo PT.  Fixed order.
+template <int THREADS, int VEC>
+__device__ __forceinline__ void norm_partials(const double (&nacc)[VEC], double* red, int PT,
+                                              double* out)
+{
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) red[threadIdx.x * VEC + i] = nacc[i];
+    __syncthreads();
+    for (int q = threadIdx.x; q < PT; q += THREADS)
+    {
+        double sum = 0.0;
+        for (int e = q; e < THREADS * VEC; e += PT) sum += red[e];
+        out[q] = sum;
+    }
+}
+
+constexpr int THREE_TERM_THREADS = 256;
+constexpr int THREE_TERM_CTAS = 3;  // per SM
+constexpr int THREE_TERM_U = 3;     // pieces in flight (four CTAs of two are as fast, but leave
+                                    // more partial sums to add; four of three spill)
+
+// Wout = W - alpha_j v_j - beta_{j-1} v_{j-1}, partials[cta][p] = |Wout|^2:
+// the whole orthogonalisation without a basis.  Bound by HBM: four vectors.
+// us a pass against the TMA ring's: 524,175 x 256 FP32 340 -> 312 (6.9 TB/s),
+// 131,072 x 128 FP32 50 -> 45, 8,192 x 256 FP32 11.0 -> 8.9, 89,999 x 128 FP64
+// 59 -> 58.
+template <typename VT>
+__global__ void __launch_bounds__(THREE_TERM_THREADS, THREE_TERM_CTAS)
+k_three_term(const StreamArgs<VT> a)
+{
+    constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+    constexpr int STEP = THREE_TERM_THREADS * VEC;  // a multiple of b (at most 1024, 512 in FP64)
+    constexpr int U = THREE_TERM_U;
+    __shared__ double red[STEP];
+    const int tid = threadIdx.x;
+    const int b = a.b;
+    pdl_wait();
+    pdl_trigger();
+    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
+    {
+        if (tid == 0) atomicExch(a.error, 1);
+        return;
+    }
+    double cj[VEC], cm[VEC], nacc[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i)
+    {
+        const int p = (tid * VEC + i) % b;
+        cj[i] = a.aj[p] * a.sj[p];
+        cm[i] = a.Vm ? a.bm[p] * a.sm[p] : 0.0;
+        nacc[i] = 0.0;
+    }
+    const VT* vm = a.Vm ? a.Vm : a.W;  // without v_{j-1}: read, not used
+    const int64_t total = a.n * b;
+    const int64_t pieces = total / STEP;
+    for (int64_t q0 = blockIdx.x; q0 < pieces; q0 += static_cast<int64_t>(U) * gridDim.x)
+    {
+        VT w[U][VEC], x[U][VEC], y[U][VEC];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int64_t q = min(q0 + static_cast<int64_t>(u) * gridDim.x, pieces - 1);
+            const int64_t o = (pieces - 1 - q) * STEP + tid * VEC;
+            load_once(a.W + o, w[u]);
+            load_once(a.Vj + o, x[u]);
+            load_once(vm + o, y[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int64_t q = q0 + static_cast<int64_t>(u) * gridDim.x;
+            if (q < pieces)
+            {
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                {
+                    double d = static_cast<double>(w[u][i]) - cj[i] * static_cast<double>(x[u][i]);
+                    if (a.Vm) d -= cm[i] * static_cast<double>(y[u][i]);
+                    w[u][i] = static_cast<VT>(d);
+                    d = static_cast<double>(w[u][i]);
+                    nacc[i] += d * d;
+                }
+                store_vec(a.Wout + (pieces - 1 - q) * STEP + tid * VEC, w[u]);
+            }
+        }
+    }
+    if (blockIdx.x == gridDim.x - 1)  // past the last whole piece
+#pragma unroll
+        for (int i = 0; i < VEC; ++i)
+        {
+            const int64_t o = pieces * STEP + tid * VEC + i;
+            if (o >= total) break;
+            double d = static_cast<double>(a.W[o]) - cj[i] * static_cast<double>(a.Vj[o]);
+            if (a.Vm) d -= cm[i] * static_cast<double>(a.Vm[o]);
+            const VT r = static_cast<VT>(d);
+            a.Wout[o] = r;
+            d = static_cast<double>(r);
+            nacc[i] += d * d;
+        }
+    norm_partials<THREE_TERM_THREADS, VEC>(nacc, red, b,
+                                           a.partials + static_cast<int64_t>(blockIdx.x) * b);
+}
+
+constexpr int REORTH_THREADS = 512;  // one CTA per SM
+constexpr int REORTH_U = 4;          // pieces per turn ..
+constexpr int REORTH_V = 4;          // .. and basis vectors in flight (128 KB per SM)
+
+// Wout = W - sum_i c_i v_i over J basis vectors, in order from the newest;
+// partials[cta][p] = |Wout|^2, and the FP16 parts of Wout (x16).  Bound by
+// HBM.  A thread holds REORTH_U pieces of w in FP64 and loads four vectors'
+// pieces at once.  Of 256 or 512 threads, one to four CTAs per SM, two or four
+// pieces and two to eight vectors this kept the most in flight without spills
+// that count.  us a pass against the TMA ring's, J = 25 unless said:
+// 262,144 x 256 FP32 1,199 -> 1,099 (6.6 TB/s), 8,192 x 256 FP32 54 -> 38,
+// 32,768 x 64 FP32 50 -> 40, 100,003 x 128 FP32 (J = 15) 154 -> 142,
+// 16,384 x 256 FP64 (J = 15) 96 -> 85, 40,009 x 64 FP64 (J = 20) 80 -> 71.
+// NARROW: fewer probes than VEC.
+template <typename VT, bool NARROW>
+__global__ void __launch_bounds__(REORTH_THREADS, 1) k_reorth(const StreamArgs<VT> a)
+{
+    constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+    constexpr int STEP = REORTH_THREADS * VEC;
+    constexpr int U = REORTH_U;
+    constexpr int V = REORTH_V;
+    __shared__ double red[STEP];
+    __shared__ __align__(16) float x16_scale[STREAM_CONSUMERS];
+    const int tid = threadIdx.x;
+    const int b = a.b;
+    const int PT = a.PT;  // probes of this CTA: b, at most 256
+    // value e of a piece: row e / PT, probe e % PT (fewer probes than VEC
+    // repeat within it; PT = b then, and the values are adjacent all the same)
+    const int RSTEP = STEP / PT;
+    const int roff = tid * VEC / PT;
+    const int pl = tid * VEC % PT;
+    const int p0 = blockIdx.y * PT;
+    pdl_wait();
+    pdl_trigger();
+    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
+    {
+        if (tid == 0) atomicExch(a.error, 1);
+        return;
+    }
+    double nacc[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) nacc[i] = 0.0;
+    // the split probe block (x16, b = 128 or 256): each probe's 2^e_p from the
+    // reduced |w|^2 partials of the dots pass (a fixed order)
+    bool x16_on = false;
+    if constexpr (sizeof(VT) == 4 && !NARROW)
+    {
+        if (a.x16 && a.wn2_in)
+        {
+            x16_on = true;
+            const int q = tid % PT;
+            const int part = tid / PT;
+            const int parts = REORTH_THREADS / PT;
+            double n2 = 0.0;
+            for (int g = part; g < a.wn2_grid; g += parts)
+                n2 += a.wn2_in[static_cast<int64_t>(g) * b + p0 + q];
+            red[tid] = n2;
+            __syncthreads();
+            if (part == 0)
+            {
+                for (int k = 1; k < parts; ++k) n2 += red[k * PT + q];
+                const int e = (n2 > 0.0 && isfinite(n2)) ? x16_exp(1.0 / sqrt(n2)) : 0;
+                x16_scale[q] = ldexpf(1.0f, e);
+                if (blockIdx.x == 0) a.x16exp[p0 + q] = e;
+            }
+            __syncthreads();
+        }
+    }
+    const VT* cf = a.coef + p0;
+    auto coefs = [&](int i, VT (&c)[VEC]) {
+        const VT* row = cf + static_cast<int64_t>(i) * b;
+        if constexpr (!NARROW)
+            load_vec(row + pl, c);
+        else
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) c[k] = row[(pl + k) % PT];
+    };
+    // pieces of 16 bytes all of which exist: the others (rows past n, pieces
+    // past the last) load a piece that does and store nothing
+    const int64_t total = a.n * b;
+    const int64_t pieces = total < VEC ? 0 : (a.n + RSTEP - 1) / RSTEP;
+    const int64_t spare = NARROW ? 0 : p0 + pl;
+    for (int64_t q0 = blockIdx.x; q0 < pieces; q0 += static_cast<int64_t>(U) * gridDim.x)
+    {
+        double w[U][VEC];
+        uint32_t o[U];  // in 16 bytes
+        unsigned int live = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int64_t q = q0 + static_cast<int64_t>(u) * gridDim.x;
+            const int64_t at = ((pieces - 1 - q) * RSTEP + roff) * b + p0 + pl;
+            const bool is = q < pieces && at + VEC <= total;
+            if (is) live |= 1u << u;
+            o[u] = static_cast<uint32_t>((is ? at : spare) / VEC);
+            VT x[VEC];
+            load_once(a.W + static_cast<uint64_t>(o[u]) * VEC, x);
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) w[u][i] = static_cast<double>(x[i]);
+        }
+        int slot = ring_slot(a.last, a.bs);
+        auto next_vector = [&]() {
+            const VT* v = a.basis + static_cast<int64_t>(slot) * a.slot_elems;
+            if (--slot < 0) slot += a.bs;
+            return v;
+        };
+        int i0 = 0;
+        for (; i0 + V <= a.J; i0 += V)
+        {
+            VT x[V][U][VEC], c[V][VEC];
+#pragma unroll
+            for (int t = 0; t < V; ++t)
+            {
+                const VT* v = next_vector();
+#pragma unroll
+                for (int u = 0; u < U; ++u) load_once(v + static_cast<uint64_t>(o[u]) * VEC, x[t][u]);
+                coefs(i0 + t, c[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < V; ++t)
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                {
+                    const double ci = static_cast<double>(c[t][i]);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) w[u][i] -= ci * static_cast<double>(x[t][u][i]);
+                }
+        }
+        for (; i0 < a.J; ++i0)
+        {
+            VT x[U][VEC], c[VEC];
+            const VT* v = next_vector();
+#pragma unroll
+            for (int u = 0; u < U; ++u) load_once(v + static_cast<uint64_t>(o[u]) * VEC, x[u]);
+            coefs(i0, c);
+#pragma unroll
+            for (int i = 0; i < VEC; ++i)
+            {
+                const double ci = static_cast<double>(c[i]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) w[u][i] -= ci * static_cast<double>(x[u][i]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (live >> u & 1)
+            {
+                VT r[VEC];
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                {
+                    r[i] = static_cast<VT>(w[u][i]);
+                    const double d = static_cast<double>(r[i]);
+                    nacc[i] += d * d;
+                }
+                store_vec(a.Wout + static_cast<uint64_t>(o[u]) * VEC, r);
+                if constexpr (sizeof(VT) == 4 && !NARROW)
+                    if (x16_on)
+                    {
+                        const float4 e = *reinterpret_cast<const float4*>(x16_scale + pl);
+                        r[0] *= e.x; r[1] *= e.y; r[2] *= e.z; r[3] *= e.w;
+                        const int64_t q = q0 + static_cast<int64_t>(u) * gridDim.x;
+                        x16_store(a.x16, (pieces - 1 - q) * RSTEP + roff, b, p0 + pl, r);
+                    }
+            }
+    }
+    if constexpr (NARROW)  // the values past the last whole 16 bytes
+    {
+        const int rest = static_cast<int>(total % VEC);
+        if (blockIdx.x == gridDim.x - 1 && tid == 0)
+            for (int i = 0; i < rest; ++i)
+            {
+                const int64_t o = total - rest + i;  // value i of a piece has probe i % b
+                double wv = static_cast<double>(a.W[o]);
+                for (int k = 0; k < a.J; ++k)
+                    wv -= static_cast<double>(cf[static_cast<int64_t>(k) * b + i % PT]) *
+                          static_cast<double>(a.basis[static_cast<int64_t>(
+                                                          ring_slot(a.last - k, a.bs)) *
+                                                          a.slot_elems + o]);
+                const VT wr = static_cast<VT>(wv);
+                const double d = static_cast<double>(wr);
+                a.Wout[o] = wr;
+                nacc[0] += i % PT == 0 ? d * d : 0.0;
+                nacc[1] += i % PT == 1 ? d * d : 0.0;
+            }
+    }
+    if (a.want_norm)
+        norm_partials<REORTH_THREADS, VEC>(
+            nacc, red, PT, a.partials + static_cast<int64_t>(blockIdx.x) * b + p0);
+}
 
 // ===========================================================================
 // Row-group SpMM.
