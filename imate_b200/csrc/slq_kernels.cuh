@@ -1812,7 +1812,8 @@ __global__ void k_init_block(int count, int b, int m, double s0,
 
 
 // ===========================================================================
-// TMA-streamed reorthogonalisation passes (sm_100a).
+// TMA-streamed inner products (sm_100a): the three-term update of w and its
+// products with J basis vectors in one pass.
 //
 // One CTA per SM: a producer warp moves tiles of T rows x PT probes of every
 // vector the pass reads into a ring of S shared-memory stages with
@@ -1820,14 +1821,18 @@ __global__ void k_init_block(int count, int b, int m, double s0,
 // consumer warps compute from the stages and release them through a second
 // mbarrier per stage.  The copy engine keeps S x 16 KB in flight per SM, so
 // the pass streams at HBM rate without registers spent on loads in flight.
+// The running sums, one per thread and basis vector, are in shared memory; the
+// ring lets a thread take one probe and many rows, so that few of them are
+// kept and each is touched once per 8 or 16 values.  Plain loads into
+// registers, which serve the update passes below better, were slower here
+// (262,144 x 256 FP32, J = 25: 1,290 us with two probes per thread, 1,355 with
+// one, against 1,178), as were sixteen consumer warps (1,361) and reading
+// every other value without the conversion unit (1,210).
 //
-// Work per row tile, in item order:
-//   dots   : W [, v_j, v_{j-1} (three-term update; written to Wout)],
-//            then the basis vectors last-i (skipping v_j, v_{j-1}, whose
-//            products come from the update registers) -> FP64 partials of
-//            <v_i, w> per (i, probe);
-//   reorth : Win, then the basis vectors last-i: w -= c_i v_i, written to
-//            Wout, FP64 partials of |w|^2.
+// Work per row tile, in item order: W [, v_j, v_{j-1} (three-term update;
+// written to Wout)], then the basis vectors last-i (skipping v_j, v_{j-1},
+// whose products come from the update registers) -> FP64 partials of <v_i, w>
+// per (i, probe).
 // Rows past the last whole tile are dealt over the CTAs with plain loads (one
 // CTA alone took 20 us for the 27 rows past 937 tiles of a 30,011-row matrix,
 // as long as the tiles took the others).
@@ -1996,7 +2001,7 @@ struct StreamArgs {
     int32_t* x16exp;
 };
 
-// The dots pass.  R = rows per consumer thread per tile.
+// R = rows per consumer thread per tile.
 template <typename VT, int R>
 __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<VT> a)
 {
@@ -2024,7 +2029,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
     // items per tile
     const bool upd = a.do_update != 0;
     const int npre = 1 + (upd ? (a.Vm ? 2 : 1) : 0);
-    // dots: basis vectors v_j, v_{j-1} are served from the update registers
+    // basis vectors v_j, v_{j-1} are served from the update registers
     const int skip = upd ? (a.Vm ? 2 : 1) : 0;
     const int nbasis = (J > skip) ? J - skip : 0;
     const int nitems = npre + nbasis;
@@ -2135,7 +2140,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                 if (*reinterpret_cast<volatile int*>(abort_flag)) { ok = false; break; }
                 if (item >= npre && item + 1 < nitems)
                 {
-                    // dots: two basis tiles per turn, four FMA chains each, so
+                    // two basis tiles per turn, four FMA chains each, so
                     // the two load -> convert -> FMA -> add-tree chains overlap
                     // (two warps per scheduler leave little else to hide them)
                     const int ib = skip + (item - npre);
@@ -2173,7 +2178,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                     ++item;
                     continue;
                 }
-                // dots: fetch this thread's running sum before the wait so the
+                // fetch this thread's running sum before the wait so the
                 // shared-memory latency overlaps it
                 const int ib = skip + (item - npre);
                 double prev = 0.0;
