@@ -1952,7 +1952,23 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     const int T = R * (STREAM_CONSUMERS / PT);
     int S = 0;
     size_t smem = 0;
-    if constexpr (MODE == 0)
+    // FP64 inner products of up to DOTS_MAX_J vectors come from plain loads
+    const bool loads = MODE == 0 && sizeof(VT) == 8 && J <= DOTS_MAX_J;
+    if (loads)
+    {
+        smem = static_cast<size_t>(std::max(J, 1)) * DOTS_THREADS * sizeof(double);
+        if constexpr (sizeof(VT) == 8)
+        {
+            static bool attr = false;
+            if (!attr)
+            {
+                SLQ_CK(cudaFuncSetAttribute(k_dots, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            DOTS_MAX_J * DOTS_THREADS * 8));
+                attr = true;
+            }
+        }
+    }
+    else if constexpr (MODE == 0)
     {
         const size_t fixed = STREAM_BARRIER_BYTES + STREAM_CONSUMERS * sizeof(double);
         const size_t extra = static_cast<size_t>(J) * STREAM_CONSUMERS * 8;
@@ -2022,7 +2038,12 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     const int writes = ((MODE == 1 || do_update) ? 1 : 0) + (x16 ? 1 : 0);
     ProfScope prof(MODE == 0 ? SLQ_K_DOTS : SLQ_K_REORTH, vb * (reads + writes), L.st);
     if constexpr (MODE == 0)
-        SLQ_TRY(launch_pdl(L.st, k_stream<VT, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
+    {
+        if constexpr (sizeof(VT) == 8)
+            if (loads) SLQ_TRY(launch_pdl(L.st, k_dots, dim3(gx, gy), DOTS_THREADS, smem, a));
+        if (!loads)
+            SLQ_TRY(launch_pdl(L.st, k_stream<VT, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
+    }
     else if (J > 0 && b * sizeof(VT) >= 16)
         SLQ_TRY(launch_pdl(L.st, k_reorth<VT, false>, dim3(gx, gy), REORTH_THREADS, 0, a));
     else if (J > 0)

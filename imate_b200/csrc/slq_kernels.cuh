@@ -2342,6 +2342,13 @@ __device__ __forceinline__ void load_once(const double* p, double (&v)[2])
                  : "l"(p));
 }
 
+__device__ __forceinline__ double load_once(const double* p)
+{
+    double v;
+    asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ void load_vec(const float* p, float (&v)[4])
 {
     const float4 x = *reinterpret_cast<const float4*>(p);
@@ -2657,6 +2664,130 @@ __global__ void __launch_bounds__(REORTH_THREADS, 1) k_reorth(const StreamArgs<V
     if (a.want_norm)
         norm_partials<REORTH_THREADS, VEC>(
             nacc, red, PT, a.partials + static_cast<int64_t>(blockIdx.x) * b + p0);
+}
+
+constexpr int DOTS_THREADS = 512;  // one CTA per SM
+constexpr int DOTS_U = 4;          // rows of a thread per turn ..
+constexpr int DOTS_V = 8;          // .. and basis vectors in flight (128 KB per SM)
+// basis vectors whose running sums (a double per thread) fit shared memory
+constexpr int DOTS_MAX_J = 48;
+
+// The FP64 pass of k_stream from plain loads: an eight-byte value per lane
+// keeps enough bytes in flight without the ring, and four rows a turn balance
+// better than its 16 KB tiles.  A thread takes one probe; rows go round the
+// CTAs.  Sums, order of the vectors and results as there; used up to
+// DOTS_MAX_J vectors.  us a pass against the ring's, mean over a run:
+// 16,384 x 256, J up to 30 101 -> 88; 40,009 x 64, J up to 40 85 -> 77 (the
+// update pass after it finds less in L2: 78 -> 82 and 68 -> 76).  FP32 is
+// slower this way, see above.
+__global__ void __launch_bounds__(DOTS_THREADS, 1) k_dots(const StreamArgs<double> a)
+{
+    constexpr int U = DOTS_U;
+    constexpr int V = DOTS_V;
+    extern __shared__ double smem_dots[];  // [max(J, 1)][DOTS_THREADS]
+    double* acc = smem_dots + threadIdx.x;
+    const int tid = threadIdx.x;
+    const int b = a.b;
+    const int PT = a.PT;
+    const int J = a.J;
+    const int RSTEP = DOTS_THREADS / PT;
+    const int pl = tid % PT;
+    const int roff = tid / PT;
+    const int p0 = blockIdx.y * PT;
+    const bool upd = a.do_update != 0;
+    // v_j, v_{j-1} are served from the update
+    const int skip = upd ? (a.Vm ? 2 : 1) : 0;
+    for (int i = 0; i < J; ++i) acc[i * DOTS_THREADS] = 0.0;
+    pdl_wait();
+    pdl_trigger();
+    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
+    {
+        if (tid == 0) atomicExch(a.error, 1);
+        return;
+    }
+    double cj = 0.0, cm = 0.0;
+    if (upd)
+    {
+        cj = a.aj[p0 + pl] * a.sj[p0 + pl];
+        cm = a.Vm ? a.bm[p0 + pl] * a.sm[p0 + pl] : 0.0;
+    }
+    const double* vm = a.Vm ? a.Vm : a.Vj;
+    const int64_t pieces = (a.n + RSTEP - 1) / RSTEP;
+    for (int64_t q0 = blockIdx.x; q0 < pieces; q0 += static_cast<int64_t>(U) * gridDim.x)
+    {
+        // rows past the last one read row 0 and count as zero
+        double w[U];
+        int64_t o[U];
+        unsigned int live = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int64_t r = (q0 + static_cast<int64_t>(u) * gridDim.x) * RSTEP + roff;
+            if (r < a.n) live |= 1u << u;
+            o[u] = (r < a.n ? r : 0) * b + p0 + pl;
+            w[u] = load_once(a.W + o[u]);
+        }
+        if (upd)
+        {
+            double x[U], y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                x[u] = load_once(a.Vj + o[u]);
+                y[u] = load_once(vm + o[u]);
+            }
+            double lj = 0.0, lm = 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                w[u] -= cj * x[u];
+                if (a.Vm) w[u] -= cm * y[u];
+                if (live >> u & 1)
+                {
+                    a.Wout[o[u]] = w[u];
+                    lj += x[u] * w[u];
+                    lm += y[u] * w[u];
+                }
+            }
+            if (J > 0) acc[0] += lj;
+            if (a.Vm && J > 1) acc[DOTS_THREADS] += lm;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (!(live >> u & 1)) w[u] = 0.0;
+        int slot = ring_slot(a.last - skip, a.bs);
+        for (int i0 = skip; i0 < J; i0 += V)
+        {
+            double x[V][U];
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                if (i0 + v < J)
+                {
+                    const double* src = a.basis + static_cast<int64_t>(slot) * a.slot_elems;
+                    if (--slot < 0) slot += a.bs;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) x[v][u] = load_once(src + o[u]);
+                }
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                if (i0 + v < J)
+                {
+                    static_assert(U == 4, "two chains of two");
+                    const double l0 = x[v][0] * w[0] + x[v][1] * w[1];
+                    const double l1 = x[v][2] * w[2] + x[v][3] * w[3];
+                    acc[(i0 + v) * DOTS_THREADS] += l0 + l1;
+                }
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < J * PT; idx += DOTS_THREADS)
+    {
+        const int i = idx / PT;
+        const int q = idx % PT;
+        double sum = 0.0;
+        for (int r = 0; r < RSTEP; ++r) sum += smem_dots[i * DOTS_THREADS + r * PT + q];
+        a.partials[(static_cast<int64_t>(blockIdx.x) * J + i) * b + p0 + q] = sum;
+    }
 }
 
 // ===========================================================================

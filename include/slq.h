@@ -259,9 +259,9 @@ slq_status slq_group_fill(int64_t n, const int32_t* indptr,
 /* Dense FP32 operator (the role of cuDenseMatrix: construction and upload
  * imate/_cu_linear_operator/cu_dense_matrix.cu:39-61 and :94-122, cuBLAS
  * gemv products :130-238): A is num_rows x num_cols, row-major, in device
- * memory.  Creation splits A (and, with need_transpose, A^T) into TF32
- * hi/lo parts in the workspace; products run on the tensor cores
- * (tcgen05 kind::tf32, three terms: ~FP32 accuracy) with the SpMM
+ * memory.  Creation splits A (and, with need_transpose, A^T) into three BF16
+ * parts (all 24 bits) in the workspace; products run on the tensor cores
+ * (tcgen05 kind::f16, six terms: ~FP32 accuracy) with the SpMM
  * epilogue.  The workspace also holds the probe-block parts of one product,
  * so an operator serves one product at a time (not two runs at once, and
  * not batch plans); the tuner does not apply to it.  Float32 only. */

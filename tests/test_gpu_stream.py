@@ -47,3 +47,15 @@ def test_rows_past_the_last_tile(cuda, block, n, orth):
                      max_num_samples=max(count, block), **kw)[:count]
         assert np.max(np.abs(got32 - ref) / np.abs(ref)) < 1e-6 * \
             max(1.0, n / np.min(np.abs(ref)))
+
+
+def test_more_vectors_than_the_sums_of_one_pass(cuda):
+    """Float64 products with more basis vectors than fit the plain-load pass
+    (48), and with more than one launch takes (64)."""
+    A = ib.correlation_matrix(211, scale=0.05, shift=0.3, seed=2)
+    kw = dict(min_num_samples=3, max_num_samples=3, error_rtol=0.0,
+              lanczos_degree=70, orthogonalize=-1, seed=3)
+    want = oracle.trace_estimator(A, "log", gram=False, **kw)
+    got = _run(ib.Matrix(A, reorder=False, group_rows=0), **kw)
+    ref = want["samples"][:3, 0]
+    assert np.max(np.abs(got - ref) / np.abs(ref)) < 1e-10
