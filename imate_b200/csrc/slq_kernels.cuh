@@ -28,6 +28,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "slq_ql.cuh"
 #include "slq_tc.cuh"
 
 namespace slq {
@@ -708,7 +709,8 @@ k_finalize(const double* __restrict__ partials, int nparts, int cols, int mode,
 // the latency of that chain and not by any unit.  A probe has a warp of its
 // own (a thread per probe made every probe of a warp wait for the slowest
 // deflation sequence), the arrays lie in shared memory with the next
-// rotation's entries loaded a rotation ahead, the search for a negligible
+// rotation's entries loaded a rotation ahead, lane 0 alone walks the chain (no
+// lane reads what another one stores), the search for a negligible
 // off-diagonal entry is one ballot, and a rotation costs one reciprocal
 // square root instead of hypot and two divisions.  The quadrature has no
 // chain: a thread per probe walked all nodes of all inquiries with a pow and
@@ -739,108 +741,6 @@ __device__ __forceinline__ double apply_func(int func, double x, const double4& 
         case 7: return 0.5 * (1.0 + tanh(c.x * x));
         default: return x;
     }
-}
-
-// Implicit QL of one warp: d, e, z in shared memory, every lane runs the
-// same chain and lane 0 stores.  Returns 1 if an eigenvalue took more than
-// 60 iterations.
-__device__ int ql_first_row(double* d, double* e, double* z, int k, int lane)
-{
-    if (k <= 1) return 0;
-    const double eps = 2.220446049250313e-16;
-    for (int l = 0; l < k; ++l)
-    {
-        int iter = 0;
-        for (;;)
-        {
-            // the first negligible off-diagonal entry from l on
-            int mm = k - 1;
-            for (int base = l; base < k - 1; base += 32)
-            {
-                const int i = base + lane;
-                const bool small =
-                    i < k - 1 && fabs(e[i]) <= eps * (fabs(d[i]) + fabs(d[i + 1]));
-                const unsigned hit = __ballot_sync(FULL_MASK, small);
-                if (hit)
-                {
-                    mm = base + __ffs(hit) - 1;
-                    break;
-                }
-            }
-            if (mm == l) break;
-            if (++iter > 60) return 1;
-            double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-            double r = fabs(g) < 1e150 ? sqrt(g * g + 1.0) : hypot(g, 1.0);
-            g = d[mm] - d[l] + e[l] / (g + (g >= 0.0 ? r : -r));
-            double s = 1.0, c = 1.0, p = 0.0;
-            bool deflated = false;
-            // zf and dh carry z[i + 1] and the old d[i + 1]; dn, en, zn are
-            // the entries of the next rotation
-            double zf = z[mm], dh = d[mm];
-            double dn = d[mm - 1], en = e[mm - 1], zn = z[mm - 1];
-            __syncwarp();
-            for (int i = mm - 1; i >= l; --i)
-            {
-                const double di = dn, ei = en, zi = zn;
-                if (i > l)
-                {
-                    dn = d[i - 1];
-                    en = e[i - 1];
-                    zn = z[i - 1];
-                }
-                const double f = s * ei;
-                const double bb = c * ei;
-                const double h = f * f + g * g;
-                if (h > 1e-280 && h < 1e280)
-                {
-                    const double q = rsqrt(h);
-                    r = h * q;
-                    s = f * q;
-                    c = g * q;
-                }
-                else
-                {
-                    // squares that would leave the range of a double
-                    r = hypot(f, g);
-                    if (r == 0.0)
-                    {
-                        if (lane == 0)
-                        {
-                            e[i + 1] = 0.0;
-                            d[i + 1] = dh - p;
-                            z[i + 1] = zf;
-                            e[mm] = 0.0;
-                        }
-                        deflated = true;
-                        break;
-                    }
-                    s = f / r;
-                    c = g / r;
-                }
-                g = dh - p;
-                const double t = (di - g) * s + 2.0 * c * bb;
-                p = s * t;
-                if (lane == 0)
-                {
-                    e[i + 1] = r;
-                    d[i + 1] = g + p;
-                    z[i + 1] = s * zi + c * zf;
-                }
-                g = c * t - bb;
-                zf = c * zi - s * zf;
-                dh = di;
-            }
-            if (!deflated && lane == 0)
-            {
-                d[l] = dh - p;
-                z[l] = zf;
-                e[l] = g;
-                e[mm] = 0.0;
-            }
-            __syncwarp();
-        }
-    }
-    return 0;
 }
 
 // theta[i][p], tau[i][p] (row stride b) for i < size[p]; status[p]: bit 1
