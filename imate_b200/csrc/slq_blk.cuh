@@ -921,7 +921,7 @@ k_spmm_blk(const BlkArgs d)
             if (row < 0) return;
             const float4* src = reinterpret_cast<const float4*>(d.X + int64_t(row) * NB) + (ct & 15);
 #pragma unroll
-            for (int j = 0; j < nj; ++j) buf[j] = __ldg(src + 16 * j);
+            for (int j = 0; j < nj; ++j) buf[j] = src[16 * j];
         };
         // the scales of this thread's probes
         float4 xs[nj];
@@ -1093,8 +1093,8 @@ k_spmm_blk(const BlkArgs d)
                 for (int q = 0; q < 4; ++q)
                 {
                     float4 x4 = make_float4(0.f, 0.f, 0.f, 0.f), z4 = x4;
-                    if (live && need_x) x4 = __ldg(reinterpret_cast<const float4*>(d.X + o) + q);
-                    if (live && need_z) z4 = __ldg(reinterpret_cast<const float4*>(d.Z + o) + q);
+                    if (live && need_x) x4 = reinterpret_cast<const float4*>(d.X + o)[q];
+                    if (live && need_z) z4 = reinterpret_cast<const float4*>(d.Z + o)[q];
                     xv[4 * q] = x4.x; xv[4 * q + 1] = x4.y; xv[4 * q + 2] = x4.z; xv[4 * q + 3] = x4.w;
                     zv[4 * q] = z4.x; zv[4 * q + 1] = z4.y; zv[4 * q + 2] = z4.z; zv[4 * q + 3] = z4.w;
                 }

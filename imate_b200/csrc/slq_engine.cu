@@ -1103,12 +1103,16 @@ struct Launcher {
     cudaStream_t st;
     int sms;
     int64_t launches = 0;
+    bool early = true;  // the next launch may overlap its predecessor
 };
 
 // A launch that may overlap its predecessor's end (programmatic stream
 // serialization): only for kernels that call pdl_wait before they touch memory.
+// The first launch of a call that follows the caller's own work in the stream
+// (L.early false) goes in stream order: that work may have written the
+// operator's arrays, which the kernels read as constant.
 template <typename... P, typename... A>
-slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+slq_status launch_pdl(Launcher& L, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                       A... args)
 {
     cudaLaunchAttribute attr{};
@@ -1118,9 +1122,10 @@ slq_status launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 blo
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
+    cfg.stream = L.st;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = L.early ? 1 : 0;
+    L.early = true;
     SLQ_CK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
     return SLQ_OK;
 }
@@ -1145,7 +1150,7 @@ slq_status spmm_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, const 
     const size_t smem = (epi != 0) ? 8 * static_cast<size_t>(b) * sizeof(double) : 0;
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>((nrows + 7) / 8, int64_t(L.sms) * 4)));
-    SLQ_TRY(launch_pdl(L.st, k_spmm<VT, LV, KS>, grid, 256, smem, ptr, ind, vals, nrows, b, X, sx,
+    SLQ_TRY(launch_pdl(L, k_spmm<VT, LV, KS>, grid, 256, smem, ptr, ind, vals, nrows, b, X, sx,
                        shift, Y, Z, zc, zs, epi, partials));
     ++L.launches;
     *grid_out = grid;
@@ -1187,7 +1192,7 @@ slq_status spmm_rows_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, c
     const int64_t want = (nrows + RW * warps - 1) / (RW * warps);
     const int grid =
         static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(L.sms) * per_sm)));
-    SLQ_TRY(launch_pdl(L.st, k_spmm_rows<VT, LPR, C, PLAIN>, grid, warps * 32,
+    SLQ_TRY(launch_pdl(L, k_spmm_rows<VT, LPR, C, PLAIN>, grid, warps * 32,
                        epi != 0 ? smem_of(warps) : 0, ptr, ind, vals, nrows, X, sx, shift, Y, Z, zc,
                        zs, epi, partials));
     ++L.launches;
@@ -1263,11 +1268,11 @@ slq_status finalize(Launcher& L, const double* partials, int nparts, int cols, i
 {
     ProfScope prof(SLQ_K_FINALIZE, double(nparts) * cols * 8.0, L.st);
     if (mode == FIN_COEF)
-        SLQ_TRY(launch_pdl(L.st, k_finalize<VT, 32, 32>, (cols + 31) / 32, 1024, 0, partials, nparts,
+        SLQ_TRY(launch_pdl(L, k_finalize<VT, 32, 32>, (cols + 31) / 32, 1024, 0, partials, nparts,
                            cols, mode, out, coef, scales, b, bs, last, next_scale, active, size,
                            check_break, thr, step));
     else
-        SLQ_TRY(launch_pdl(L.st, k_finalize<VT, 8, 64>, (cols + 7) / 8, 512, 0, partials, nparts,
+        SLQ_TRY(launch_pdl(L, k_finalize<VT, 8, 64>, (cols + 7) / 8, 512, 0, partials, nparts,
                            cols, mode, out, coef, scales, b, bs, last, next_scale, active, size,
                            check_break, thr, step));
     ++L.launches;
@@ -1455,7 +1460,7 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
         const int grid = grid_all;
         const int64_t pad = round_up(K, DT_BK);
         dim3 tg(static_cast<unsigned>((pad + 63) / 64), static_cast<unsigned>((nb + 31) / 32));
-        SLQ_TRY(launch_pdl(L.st, k_dense_split_t, tg, dim3(32, 8), 0, X, K, int64_t(b),
+        SLQ_TRY(launch_pdl(L, k_dense_split_t, tg, dim3(32, 8), 0, X, K, int64_t(b),
                            int64_t(p_off), int64_t(nb), pad, op->ldx, 256 * op->ldx,
                            op->xt_parts));
         ++L.launches;
@@ -1485,13 +1490,13 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
         d.error = error ? error : op->d_error;
         d.ksplit = ksplit;
         d.acc = op->d_acc;
-        SLQ_TRY(launch_pdl(L.st, k_dense_tc, grid, DT_THREADS, dense_smem(NB), a_parts, x_parts, d));
+        SLQ_TRY(launch_pdl(L, k_dense_tc, grid, DT_THREADS, dense_smem(NB), a_parts, x_parts, d));
         ++L.launches;
         if (ksplit > 1)
         {
             int CP = 32;
             while (CP < nb) CP <<= 1;
-            SLQ_TRY(launch_pdl(L.st, k_dense_epi, epi_grid, 256, 0, d, CP));
+            SLQ_TRY(launch_pdl(L, k_dense_epi, epi_grid, 256, 0, d, CP));
             ++L.launches;
         }
     }
@@ -1563,7 +1568,7 @@ slq_status spmm_rg_inst(Launcher& L, const int32_t* gptr, const int32_t* gcol, c
     const size_t smem = epi != 0 ? static_cast<size_t>(per_cta) * b * sizeof(double) : 0;
     const int grid = static_cast<int>(std::max<int64_t>(
         1, std::min<int64_t>((items + per_cta - 1) / per_cta, int64_t(L.sms) * per_sm)));
-    SLQ_TRY(launch_pdl(L.st, k_spmm_rg<VT, LPR, RPW, PLAIN>, grid, warps * 32, smem, gptr, gcol,
+    SLQ_TRY(launch_pdl(L, k_spmm_rg<VT, LPR, RPW, PLAIN>, grid, warps * 32, smem, gptr, gcol,
                        gval, nrows, ng, G, b, X, sx, shift, Y, Z, zc, zs, epi, partials));
     ++L.launches;
     *grid_out = grid;
@@ -1710,13 +1715,13 @@ slq_status spmm_blk_inst(Launcher& L, const slq_op* op, int transpose, int b, co
     d.x16 = pre ? maps->x16 : nullptr;
     d.xexp = ready ? maps->x16exp : nullptr;
     if (pre && b == 256)
-        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<256, true>, grid, BLK_THREADS, smem, d));
+        SLQ_TRY(launch_pdl(L, k_spmm_blk<256, true>, grid, BLK_THREADS, smem, d));
     else if (pre)
-        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<128, true>, grid, BLK_THREADS, smem, d));
+        SLQ_TRY(launch_pdl(L, k_spmm_blk<128, true>, grid, BLK_THREADS, smem, d));
     else if (b == 256)
-        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<256, false>, grid, BLK_THREADS, smem, d));
+        SLQ_TRY(launch_pdl(L, k_spmm_blk<256, false>, grid, BLK_THREADS, smem, d));
     else
-        SLQ_TRY(launch_pdl(L.st, k_spmm_blk<128, false>, grid, BLK_THREADS, smem, d));
+        SLQ_TRY(launch_pdl(L, k_spmm_blk<128, false>, grid, BLK_THREADS, smem, d));
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -2040,16 +2045,16 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     if constexpr (MODE == 0)
     {
         if constexpr (sizeof(VT) == 8)
-            if (loads) SLQ_TRY(launch_pdl(L.st, k_dots, dim3(gx, gy), DOTS_THREADS, smem, a));
+            if (loads) SLQ_TRY(launch_pdl(L, k_dots, dim3(gx, gy), DOTS_THREADS, smem, a));
         if (!loads)
-            SLQ_TRY(launch_pdl(L.st, k_stream<VT, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
+            SLQ_TRY(launch_pdl(L, k_stream<VT, R>, dim3(gx, gy), STREAM_THREADS, smem, a));
     }
     else if (J > 0 && b * sizeof(VT) >= 16)
-        SLQ_TRY(launch_pdl(L.st, k_reorth<VT, false>, dim3(gx, gy), REORTH_THREADS, 0, a));
+        SLQ_TRY(launch_pdl(L, k_reorth<VT, false>, dim3(gx, gy), REORTH_THREADS, 0, a));
     else if (J > 0)
-        SLQ_TRY(launch_pdl(L.st, k_reorth<VT, true>, dim3(gx, gy), REORTH_THREADS, 0, a));
+        SLQ_TRY(launch_pdl(L, k_reorth<VT, true>, dim3(gx, gy), REORTH_THREADS, 0, a));
     else
-        SLQ_TRY(launch_pdl(L.st, k_three_term<VT>, gx, THREE_TERM_THREADS, 0, a));
+        SLQ_TRY(launch_pdl(L, k_three_term<VT>, gx, THREE_TERM_THREADS, 0, a));
     ++L.launches;
     *grid_out = gx;
     return SLQ_OK;
@@ -2255,7 +2260,7 @@ slq_status launch_probes(Launcher& L, const RunPlan& r, int rng, int64_t seed, i
     {
         const dim3 grid(static_cast<unsigned>((r.b + PROBE_TILE - 1) / PROBE_TILE),
                         static_cast<unsigned>(r.nchunks));
-        SLQ_TRY(launch_pdl(L.st, k_probe_parity<VT>, grid, 256, 0, r.nv, r.b, count, r.wpp, r.cw,
+        SLQ_TRY(launch_pdl(L, k_probe_parity<VT>, grid, 256, 0, r.nv, r.b, count, r.wpp, r.cw,
                            B.starts, B.chunk_polys, B.chunk_polys + PROBE_FAN * 4, inv, X));
     }
     else
@@ -2275,12 +2280,12 @@ slq_status launch_quadrature(Launcher& L, const RunPlan& r, const slq_params* p,
                              int count, double* samples, int32_t* status)
 {
     ProfScope prof(SLQ_K_EIG, double(r.m) * r.b * 16.0 + double(count) * r.q * 8.0, L.st);
-    SLQ_TRY(launch_pdl(L.st, k_ql, count, 32, 3 * sizeof(double) * r.m, r.b, r.m, B.alpha, B.beta,
+    SLQ_TRY(launch_pdl(L, k_ql, count, 32, 3 * sizeof(double) * r.m, r.b, r.m, B.alpha, B.beta,
                        B.size, r.gram == 1, B.theta, B.tau, status));
     ++L.launches;
     const int64_t pairs = int64_t(count) * r.q;
     const int grid = static_cast<int>(std::min<int64_t>((pairs + 7) / 8, int64_t(L.sms) * 8));
-    SLQ_TRY(launch_pdl(L.st, k_quad, grid, 256, 0, count, r.b, r.m, B.size, B.theta, B.tau, p->func,
+    SLQ_TRY(launch_pdl(L, k_quad, grid, 256, 0, count, r.b, r.m, B.size, B.theta, B.tau, p->func,
                        func_coeff(p), p->exponent, B.params, r.q, static_cast<double>(r.nv), samples,
                        status));
     ++L.launches;
@@ -2605,7 +2610,7 @@ slq_status run_typed(slq_op* op, const slq_params* p, const double* parameters, 
             // the block
             const uint64_t* adv = B.chunk_polys + jump_table_words(r.nchunks);
             const ulonglong4 s0v = make_ulonglong4(cur[0], cur[1], cur[2], cur[3]);
-            SLQ_TRY(launch_pdl(st, k_probe_starts, (count + 31) / 32, 32, 0, count, s0v, adv,
+            SLQ_TRY(launch_pdl(L, k_probe_starts, (count + 31) / 32, 32, 0, count, s0v, adv,
                                adv + PROBE_FAN * 4, B.starts));
             ++L.launches;
             if (g + b < max_s)
@@ -3347,6 +3352,7 @@ extern "C" slq_status slq_operator_dot(slq_op* op, int transpose, double t, cons
         return fail(SLQ_ERR_BAD_ARG, "operator_dot: operator has no transpose");
     Launcher L;
     L.st = static_cast<cudaStream_t>(stream);
+    L.early = false;
     SLQ_TRY(device_sms(&L.sms));
     const double shift = op->affine ? t : 0.0;
     int grid = 0;

@@ -71,7 +71,8 @@ __device__ __forceinline__ void load_n(const VT* p, VT (&v)[N])
     }
 }
 
-// read-only path for gathers from a buffer no thread of the kernel writes
+// read-only path: for arrays that nothing writes while the kernel is resident
+// (the operator's), see pdl_wait
 template <typename VT, int N>
 __device__ __forceinline__ void ldg_n(const VT* p, VT (&v)[N])
 {
@@ -142,6 +143,12 @@ __device__ __forceinline__ void store_n(VT* p, const VT (&v)[N])
 // completed and its writes are visible.  Since each one waits, a kernel's
 // completion implies that of all before it.  Without the launch attribute
 // both are no-ops.  What it saves is the launch gap between small kernels.
+//
+// Such a kernel is resident while its predecessor still writes the probe block,
+// scales, coefficients and partial sums, so it reads these with plain loads:
+// __ldg and `const __restrict__` parameters promise data that is constant
+// while the kernel is resident, and the compiler may move such loads above the
+// wait.  They are for the operator's arrays.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger()
 {
@@ -186,9 +193,9 @@ template <typename VT, int LV, int KS>
 __global__ void __launch_bounds__(256, SpmmOcc<VT, LV>::MINB)
 k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
        const VT* __restrict__ vals, int64_t nrows, int b,
-       const VT* __restrict__ X, const double* __restrict__ sx, double shift,
-       VT* __restrict__ Y, const VT* __restrict__ Z,
-       const double* __restrict__ zc, const double* __restrict__ zs, int epi,
+       const VT* X, const double* sx, double shift,
+       VT* __restrict__ Y, const VT* Z,
+       const double* zc, const double* zs, int epi,
        double* __restrict__ partials)
 {
     constexpr int P = 32 / KS;
@@ -242,7 +249,7 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                 VT x[4][LV];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    ldg_n<VT, LV>(X + static_cast<int64_t>(cc[u]) * b + p0, x[u]);
+                    load_n<VT, LV>(X + static_cast<int64_t>(cc[u]) * b + p0, x[u]);
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -256,7 +263,7 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                 if (src < cnt)
                 {
                     VT x[LV];
-                    ldg_n<VT, LV>(X + static_cast<int64_t>(cc) * b + p0, x);
+                    load_n<VT, LV>(X + static_cast<int64_t>(cc) * b + p0, x);
 #pragma unroll
                     for (int v = 0; v < LV; ++v) acc[v] += aa * x[v];
                 }
@@ -274,17 +281,17 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
         {
             const int64_t o = row * b + p0;
             VT xr[LV], zr[LV], yr[LV];
-            if (shift != 0.0 || epi == 1) ldg_n<VT, LV>(X + o, xr);
-            if (Z) ldg_n<VT, LV>(Z + o, zr);
+            if (shift != 0.0 || epi == 1) load_n<VT, LV>(X + o, xr);
+            if (Z) load_n<VT, LV>(Z + o, zr);
 #pragma unroll
             for (int v = 0; v < LV; ++v)
             {
                 // per-probe scales from L1 (not held in registers)
-                const double sxv = sx ? __ldg(sx + p0 + v) : 1.0;
+                const double sxv = sx ? sx[p0 + v] : 1.0;
                 double y = static_cast<double>(acc[v]) * sxv;
                 if (shift != 0.0)
                     y += shift * (sxv * static_cast<double>(xr[v]));
-                if (Z) y -= (__ldg(zc + p0 + v) * __ldg(zs + p0 + v)) * static_cast<double>(zr[v]);
+                if (Z) y -= (zc[p0 + v] * zs[p0 + v]) * static_cast<double>(zr[v]);
                 yr[v] = static_cast<VT>(y);
                 const double ys = static_cast<double>(yr[v]);
                 if (epi == 1)
@@ -399,7 +406,7 @@ __device__ __forceinline__ void finish_piece(const VT* acc, size_t o, int p0, co
     VT xr[VEC], yr[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) xr[v] = VT(0);
-    if ((!PLAIN && shift != 0.0) || epi == 1) ldg_n<VT, VEC>(X + o, xr);
+    if ((!PLAIN && shift != 0.0) || epi == 1) load_n<VT, VEC>(X + o, xr);
     if constexpr (PLAIN)
     {
 #pragma unroll
@@ -437,14 +444,14 @@ __device__ __forceinline__ void finish_piece(const VT* acc, size_t o, int p0, co
         VT zr[VEC];
 #pragma unroll
         for (int v = 0; v < VEC; ++v) zr[v] = VT(0);
-        if (Z) ldg_n<VT, VEC>(Z + o, zr);
+        if (Z) load_n<VT, VEC>(Z + o, zr);
 #pragma unroll
         for (int v = 0; v < VEC; ++v)
         {
             const double s = sxr[v];
             double y = static_cast<double>(acc[v]) * s;
             if (shift != 0.0) y += shift * (s * static_cast<double>(xr[v]));
-            if (Z) y -= (__ldg(zc + p0 + v) * __ldg(zs + p0 + v)) * static_cast<double>(zr[v]);
+            if (Z) y -= (zc[p0 + v] * zs[p0 + v]) * static_cast<double>(zr[v]);
             yr[v] = static_cast<VT>(y);
             const double ys = static_cast<double>(yr[v]);
             if (epi == 1)
@@ -471,10 +478,10 @@ struct SpmmRowsShape {
 template <typename VT, int LPR, int C, bool PLAIN>
 __global__ void __launch_bounds__(256, SpmmRowsShape<VT, C>::MINB)
 k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-            const VT* __restrict__ vals, uint32_t nrows, const VT* __restrict__ X,
-            const double* __restrict__ sx, double shift, VT* __restrict__ Y,
-            const VT* __restrict__ Z, const double* __restrict__ zc,
-            const double* __restrict__ zs, int epi, double* __restrict__ partials)
+            const VT* __restrict__ vals, uint32_t nrows, const VT* X,
+            const double* sx, double shift, VT* __restrict__ Y,
+            const VT* Z, const double* zc,
+            const double* zs, int epi, double* __restrict__ partials)
 {
     constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
     constexpr int RW = 32 / LPR;          // rows per warp
@@ -538,7 +545,7 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
                 for (int q = 0; q < C; ++q)
                 {
                     VT piece[VEC];
-                    ldg_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
+                    load_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) x[u][q * VEC + v] = piece[v];
                 }
@@ -574,7 +581,7 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) piece[v] = VT(0);
                     if (u < cnt)
-                        ldg_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
+                        load_n<VT, VEC>(Xl + static_cast<size_t>(cc[u]) * b + q * LPR * VEC, piece);
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) x[u][q * VEC + v] = piece[v];
                 }
@@ -629,9 +636,9 @@ enum { FIN_STORE = 0, FIN_COEF = 1, FIN_NORM = 2 };
 
 template <typename VT, int CW, int RL>
 __global__ void __launch_bounds__(CW * RL)
-k_finalize(const double* __restrict__ partials, int nparts, int cols, int mode,
+k_finalize(const double* partials, int nparts, int cols, int mode,
            double* __restrict__ out, VT* __restrict__ coef,
-           const double* __restrict__ scales, int b, int bs, int last,
+           const double* scales, int b, int bs, int last,
            double* __restrict__ next_scale, int32_t* __restrict__ active,
            int32_t* __restrict__ size, int check_break, double thr, int step)
 {
@@ -747,8 +754,8 @@ __device__ __forceinline__ double apply_func(int func, double x, const double4& 
 // non-finite coefficients or eigen-solve results, bit 2 QL did not converge.
 // One warp per block, 3 m doubles of shared memory.
 __global__ void __launch_bounds__(32)
-k_ql(int b, int m, const double* __restrict__ alpha, const double* __restrict__ beta,
-     const int32_t* __restrict__ size, int gram, double* __restrict__ theta,
+k_ql(int b, int m, const double* alpha, const double* beta,
+     const int32_t* size, int gram, double* __restrict__ theta,
      double* __restrict__ tau, int32_t* __restrict__ status)
 {
     extern __shared__ double smem_ql[];
@@ -796,9 +803,9 @@ k_ql(int b, int m, const double* __restrict__ alpha, const double* __restrict__ 
 // log, a zero node under 1/x) and 8 (a non-finite sample).  One warp per
 // (probe, inquiry); the sum over the nodes has a fixed order.
 __global__ void __launch_bounds__(256)
-k_quad(int count, int b, int m, const int32_t* __restrict__ size,
-       const double* __restrict__ theta, const double* __restrict__ tau, int func, double4 fc,
-       double exponent, const double* __restrict__ params, int q, double nscale,
+k_quad(int count, int b, int m, const int32_t* size,
+       const double* theta, const double* tau, int func, double4 fc,
+       double exponent, const double* params, int q, double nscale,
        double* __restrict__ samples, int32_t* __restrict__ status)
 {
     pdl_wait();
@@ -858,12 +865,12 @@ __device__ __forceinline__ uint64_t xoshiro_next_dev(uint64_t* s)
 }
 
 // s <- q(T) s for the polynomial q (4 words): 256 draws
-__device__ __forceinline__ void xoshiro_apply(uint64_t* s, const uint64_t* __restrict__ q)
+__device__ __forceinline__ void xoshiro_apply(uint64_t* s, const uint64_t* q)
 {
     uint64_t acc[4] = {0, 0, 0, 0};
     for (int w = 0; w < 4; ++w)
     {
-        uint64_t bits = __ldg(q + w);
+        uint64_t bits = q[w];
 #pragma unroll 4
         for (int i = 0; i < 64; ++i, bits >>= 1)
         {
@@ -885,8 +892,8 @@ constexpr int PROBE_FAN = 16;
 // starts[p] = the stream state s0 advanced by p probes (tables lo, hi of the
 // advance between probes)
 __global__ void __launch_bounds__(32)
-k_probe_starts(int count, ulonglong4 s0, const uint64_t* __restrict__ lo,
-               const uint64_t* __restrict__ hi, uint64_t* __restrict__ starts)
+k_probe_starts(int count, ulonglong4 s0, const uint64_t* lo,
+               const uint64_t* hi, uint64_t* __restrict__ starts)
 {
     pdl_wait();
     pdl_trigger();
@@ -916,8 +923,8 @@ constexpr int PROBE_WORDS = 16;
 template <typename VT>
 __global__ void __launch_bounds__(256)
 k_probe_parity(int64_t len, int b, int count, int64_t wpp, int cw,
-               const uint64_t* __restrict__ starts, const uint64_t* __restrict__ lo,
-               const uint64_t* __restrict__ hi, const int32_t* __restrict__ inv,
+               const uint64_t* starts, const uint64_t* lo,
+               const uint64_t* hi, const int32_t* __restrict__ inv,
                VT* __restrict__ X)
 {
     __shared__ uint64_t words[PROBE_WORDS][PROBE_TILE];
@@ -2795,9 +2802,9 @@ template <typename VT, int LPR, int RPW, bool PLAIN>
 __global__ void __launch_bounds__(256, RgShape<VT, RPW>::MINB)
 k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
           const VT* __restrict__ gval, uint32_t nrows, uint32_t ngroups, int G, int b,
-          const VT* __restrict__ X, const double* __restrict__ sx, double shift,
-          VT* __restrict__ Y, const VT* __restrict__ Z, const double* __restrict__ zc,
-          const double* __restrict__ zs, int epi, double* __restrict__ partials)
+          const VT* X, const double* sx, double shift,
+          VT* __restrict__ Y, const VT* Z, const double* zc,
+          const double* zs, int epi, double* __restrict__ partials)
 {
     constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
     constexpr int RW = 32 / LPR;          // items per warp
@@ -2867,7 +2874,7 @@ k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
         {
             VT x[U][VEC], aa[U][RPW];
 #pragma unroll
-            for (int u = 0; u < U; ++u) ldg_n<VT, VEC>(Xl + static_cast<size_t>(nc[u]) * b, x[u]);
+            for (int u = 0; u < U; ++u) load_n<VT, VEC>(Xl + static_cast<size_t>(nc[u]) * b, x[u]);
             if (k + 2 * U <= k1)
 #pragma unroll
                 for (int u = 0; u < U; ++u) nc[u] = __ldg(gcol + k + U + u);
@@ -2884,7 +2891,7 @@ k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
         for (; k < k1; ++k, val += G)
         {
             VT x[VEC], aa[RPW];
-            ldg_n<VT, VEC>(Xl + static_cast<size_t>(__ldg(gcol + k)) * b, x);
+            load_n<VT, VEC>(Xl + static_cast<size_t>(__ldg(gcol + k)) * b, x);
             ldg_n<VT, RPW>(val, aa);
 #pragma unroll
             for (int r = 0; r < RPW; ++r)
@@ -3680,7 +3687,7 @@ __global__ void k_dense_split(const float* __restrict__ A, int64_t rows, int64_t
 // out[j * ldo + r] = the parts (part elements apart) of src[r * lds + col0 +
 // j] for j < ncols, zero for rows <= r < pad (pad, ldo even).  64 x 32 tiles
 // through shared memory; block 32 x 8, lane = two adjacent r.
-__global__ void k_dense_split_t(const float* __restrict__ src, int64_t rows, int64_t lds,
+__global__ void k_dense_split_t(const float* src, int64_t rows, int64_t lds,
                                 int64_t col0, int64_t ncols, int64_t pad, int64_t ldo,
                                 int64_t part, __nv_bfloat16* __restrict__ out)
 {
