@@ -30,6 +30,7 @@
 #include "../../include/slq.h"
 #include "slq_blk.cuh"
 #include "slq_kernels.cuh"
+#include "slq_once.h"
 #include "slq_rng.h"
 
 using namespace slq;
@@ -106,6 +107,21 @@ slq_status device_sms(int* sms)
         SLQ_CK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
     }
     *sms = g_num_sms;
+    return SLQ_OK;
+}
+
+// Lets a kernel use `bytes` of dynamic shared memory on the current device (the
+// same number every time; launches past 48 KB need it).
+template <auto Kernel>
+slq_status allow_smem(size_t bytes)
+{
+    static DeviceOnce once;
+    int dev = 0;
+    SLQ_CK(cudaGetDevice(&dev));
+    SLQ_CK(static_cast<cudaError_t>(once(dev, [&] {
+        return static_cast<int>(cudaFuncSetAttribute(
+            Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    })));
     return SLQ_OK;
 }
 
@@ -1171,10 +1187,7 @@ slq_status spmm_rows_inst(Launcher& L, const int32_t* ptr, const int32_t* ind, c
     constexpr int b = LPR * C * (16 / static_cast<int>(sizeof(VT)));
     ProfScope prof(SLQ_K_SPMM, spmm_bytes<VT>(nnz, nrows, xrows, b, Z != nullptr), L.st);
     auto smem_of = [&](int warps) { return static_cast<size_t>(warps) * RW * b * sizeof(double); };
-    if (smem_of(8) > 48 * 1024)
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_rows<VT, LPR, C, PLAIN>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem_of(8))));
+    if (smem_of(8) > 48 * 1024) SLQ_TRY((allow_smem<k_spmm_rows<VT, LPR, C, PLAIN>>(smem_of(8))));
     static std::atomic<int> resident{0};
     int per_sm = resident.load();
     if (per_sm == 0)
@@ -1432,13 +1445,7 @@ slq_status dense_spmm(Launcher& L, const slq_op* op, int transpose, int b, const
     // split K when the row tiles leave most SMs idle (the same choice as the
     // scratch was sized for)
     const int ksplit = op->d_acc ? dense_ksplit(M, K, op->dense_sms) : 1;
-    static bool attr = false;
-    if (!attr)
-    {
-        SLQ_CK(cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    232448));
-        attr = true;
-    }
+    SLQ_TRY(allow_smem<k_dense_tc>(232448));
     const double bytes = double(M) * K * 6.0 + double(K) * b * 4.0 + double(M) * b * 4.0;
     ProfScope prof(SLQ_K_SPMM, bytes, L.st);
     // one grid for every chunk (the finalize reads the same partial rows for
@@ -1517,13 +1524,7 @@ slq_status spmm_rgt_inst(Launcher& L, const CUtensorMap* xmap, const int32_t* gp
                          double(nrows) * b * 4.0 * (Z ? 2.0 : 1.0);
     ProfScope prof(SLQ_K_SPMM, bytes, L.st);
     constexpr size_t smem = RgtShape<G>::SMEM;
-    static bool attr = false;
-    if (!attr)
-    {
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_rgt<G, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
-        attr = true;
-    }
+    SLQ_TRY((allow_smem<k_spmm_rgt<G, NS>>(smem)));
     const int64_t ng = (nrows + G - 1) / G;
     constexpr int GPC = RgtShape<G>::WARPS / NS;
     const int grid = static_cast<int>(
@@ -1613,13 +1614,7 @@ slq_status spmm_tc_inst(Launcher& L, const CUtensorMap* xmap, const int32_t* gpt
     const int64_t ng = (nrows + 15) / 16;
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>(ng * NS, int64_t(L.sms) * 2)));
-    static bool attr = false;
-    if (!attr)
-    {
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_tc<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(TC_DYN_SMEM)));
-        attr = true;
-    }
+    SLQ_TRY(allow_smem<k_spmm_tc<NS>>(TC_DYN_SMEM));
     k_spmm_tc<NS><<<grid, TC_THREADS, TC_DYN_SMEM, L.st>>>(*xmap, gptr, gcol, gval, nrows, ng, b,
                                                           X, sx, shift, Y, Z, zc, zs, epi,
                                                           partials, error);
@@ -1657,23 +1652,6 @@ slq_status spmm_blk_inst(Launcher& L, const slq_op* op, int transpose, int b, co
     }
     ProfScope prof(SLQ_K_SPMM, bytes, L.st);
     const size_t smem = blk_smem_bytes(b);
-    static bool attr = false;
-    if (!attr)
-    {
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_blk<128, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(blk_smem_bytes(128))));
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_blk<256, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(blk_smem_bytes(256))));
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_blk<128, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(blk_smem_bytes(128))));
-        SLQ_CK(cudaFuncSetAttribute(k_spmm_blk<256, true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(blk_smem_bytes(256))));
-        attr = true;
-    }
 
     const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(nblk, L.sms)));
     // an X without probe scales: its per-probe maxima first (into the
@@ -1714,14 +1692,17 @@ slq_status spmm_blk_inst(Launcher& L, const slq_op* op, int transpose, int b, co
     d.error = error;
     d.x16 = pre ? maps->x16 : nullptr;
     d.xexp = ready ? maps->x16exp : nullptr;
-    if (pre && b == 256)
-        SLQ_TRY(launch_pdl(L, k_spmm_blk<256, true>, grid, BLK_THREADS, smem, d));
-    else if (pre)
-        SLQ_TRY(launch_pdl(L, k_spmm_blk<128, true>, grid, BLK_THREADS, smem, d));
-    else if (b == 256)
-        SLQ_TRY(launch_pdl(L, k_spmm_blk<256, false>, grid, BLK_THREADS, smem, d));
-    else
-        SLQ_TRY(launch_pdl(L, k_spmm_blk<128, false>, grid, BLK_THREADS, smem, d));
+#define SLQ_BLK_CASE(NB, PRE)                                                       \
+    if (b == NB && pre == PRE)                                                      \
+    {                                                                               \
+        SLQ_TRY((allow_smem<k_spmm_blk<NB, PRE>>(smem)));                           \
+        SLQ_TRY(launch_pdl(L, k_spmm_blk<NB, PRE>, grid, BLK_THREADS, smem, d));    \
+    }
+    SLQ_BLK_CASE(256, true)
+    SLQ_BLK_CASE(128, true)
+    SLQ_BLK_CASE(256, false)
+    SLQ_BLK_CASE(128, false)
+#undef SLQ_BLK_CASE
     ++L.launches;
     *grid_out = grid;
     return SLQ_OK;
@@ -1963,15 +1944,7 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     {
         smem = static_cast<size_t>(std::max(J, 1)) * DOTS_THREADS * sizeof(double);
         if constexpr (sizeof(VT) == 8)
-        {
-            static bool attr = false;
-            if (!attr)
-            {
-                SLQ_CK(cudaFuncSetAttribute(k_dots, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            DOTS_MAX_J * DOTS_THREADS * 8));
-                attr = true;
-            }
-        }
+            SLQ_TRY(allow_smem<k_dots>(DOTS_MAX_J * DOTS_THREADS * sizeof(double)));
     }
     else if constexpr (MODE == 0)
     {
@@ -1982,14 +1955,7 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
         S = static_cast<int>(std::min<size_t>(STREAM_RING_BYTES / TILE,
                                               (SMEM_MAX - fixed - extra) / TILE));
         smem = fixed + static_cast<size_t>(S) * TILE + extra;
-        static bool attr = false;
-        if (!attr)
-        {
-            SLQ_CK(cudaFuncSetAttribute(k_stream<VT, R>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(SMEM_MAX)));
-            attr = true;
-        }
+        SLQ_TRY((allow_smem<k_stream<VT, R>>(SMEM_MAX)));
     }
     StreamArgs<VT> a;
     a.n = n;

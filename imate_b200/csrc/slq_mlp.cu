@@ -18,6 +18,7 @@
 #include <string>
 
 #include "../../include/slq.h"
+#include "slq_once.h"
 
 namespace {
 
@@ -253,16 +254,21 @@ size_t step_smem() { return sizeof(StepSmem); }
 
 slq_status set_smem_attr()
 {
-    static bool done = false;
-    if (done) return SLQ_OK;
+    static slq::DeviceOnce once;
     const int bytes = static_cast<int>(step_smem());
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         bytes);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = static_cast<cudaError_t>(once(dev, [&] {
+            cudaError_t s = cudaFuncSetAttribute(
+                k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (s == cudaSuccess)
+                s = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         bytes);
+            return static_cast<int>(s);
+        }));
     if (e != cudaSuccess)
         return mlp_fail(SLQ_ERR_CUDA, std::string("mlp smem attribute: ") + cudaGetErrorString(e));
-    done = true;
     return SLQ_OK;
 }
 
