@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "slq_ql.cuh"
+#include "slq_scale.cuh"
 #include "slq_tc.cuh"
 
 namespace slq {
@@ -336,12 +337,14 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
 //   entries are gathered at once, and the next row's bounds load a row ahead;
 // * the FP32 epilogue keeps off the FP64 conversion unit (16 values per clock
 //   and SM, four conversions per element before, one now): see y_scaled and
-//   f64_of_basis.
+//   f64_of_finite.  What these do not serve shows as a value that is not
+//   finite, and the thread does its rows again in FP64 (redo_rows).
 // LPR = min(32, b / VEC) lanes serve a row, 32 / LPR rows share a warp, C =
 // b / (VEC LPR) pieces per lane.
 // Measured (the 8-wide-lane k_spmm before, this kernel now), us per product:
-// 524,175 rows of 5 entries, b = 256, FP32: 575 -> 297 (X and Y alone: 165 at
-// the copy rate); 89,999 rows of 5, b = 128, FP64: 102 -> 56; 16,384 rows of
+// 524,175 rows of 5 entries, b = 256, FP32: 575 -> 308 (X and Y alone: 165 at
+// the copy rate; 294 without the looks for what the FP32 forms do not serve,
+// 340 with a branch for every piece instead of redo_rows); 89,999 rows of 5, b = 128, FP64: 102 -> 56; 16,384 rows of
 // 2, b = 256, FP64, both directions: 58 -> 33; a 524,288 x 131,072 matrix
 // with 16 random entries per column, b = 128, FP32, mean of A and A^T:
 // 216 -> 172.
@@ -357,37 +360,16 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes, int la
         asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
 }
 
-// x * s rounded to FP32, for s given as the FP32 pair sh + sl: the FP32
-// product and its exact remainder, which is the double product rounded to
-// FP32 up to ties (relative error before the rounding 2^-48).
-__device__ __forceinline__ float y_scaled(float x, float sh, float sl)
-{
-    const float p = x * sh;
-    return p + fmaf(x, sl, fmaf(x, sh, -p));
-}
-
-// 2^-896 x as a double, from the bits of x: exact for every finite x, zeros
-// and subnormals included (the FP32 exponent is read with the FP64 bias).  An
-// infinity or NaN becomes a finite value: only for a Krylov basis vector,
-// whose non-finite entries have already made the norm it was divided by
-// non-finite.
-__device__ __forceinline__ double f64_of_basis(float x)
-{
-    const int b = __float_as_int(x);
-    return __hiloint2double((b >> 3) & 0x8fffffff, b << 29);
-}
-constexpr double TWO_896 = 0x1p896;
-
 // The per-probe scales of a lane's C x VEC probes: s_p, or for FP32 products
-// without shift and Z (PLAIN) s_p as an FP32 pair in the same registers.
+// without shift and Z (PLAIN) the FP32 pair of s_p in the same registers.
 template <typename VT, bool PLAIN>
 __device__ __forceinline__ double pack_scale(double s)
 {
     if constexpr (sizeof(VT) == 4 && PLAIN)
     {
-        const float sh = static_cast<float>(s);
-        const float sl = isinf(sh) ? 0.0f : static_cast<float>(s - static_cast<double>(sh));
-        return __hiloint2double(__float_as_int(sh), __float_as_int(sl));
+        float hi, lo;
+        scale_pair(s, hi, lo);
+        return __hiloint2double(__float_as_int(hi), __float_as_int(lo));
     }
     else
         return s;
@@ -396,47 +378,55 @@ __device__ __forceinline__ double pack_scale(double s)
 // One 16-byte piece of a finished row: y = s acc [+ t s x] [- zc zs z] stored
 // at Y + o, its partial-sum term added to part (the per-probe factor s_p or
 // zs_p of the terms is applied to the sums).  p0 = the piece's first probe.
+// Where the FP32 forms do not serve the piece, part is no longer finite, and
+// without partial sums (epi 0) `redo` is set.
 template <typename VT, bool PLAIN, int VEC = 16 / static_cast<int>(sizeof(VT))>
 __device__ __forceinline__ void finish_piece(const VT* acc, size_t o, int p0, const double* sxr,
                                              bool scaled, double shift, const VT* X, VT* Y,
                                              const VT* Z, const double* zc, const double* zs,
-                                             int epi, double* part)
+                                             int epi, double* part, bool& redo)
 {
-    constexpr bool F32 = sizeof(VT) == 4;
     VT xr[VEC], yr[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) xr[v] = VT(0);
     if ((!PLAIN && shift != 0.0) || epi == 1) load_n<VT, VEC>(X + o, xr);
-    if constexpr (PLAIN)
+    if constexpr (PLAIN && sizeof(VT) == 4)
     {
 #pragma unroll
         for (int v = 0; v < VEC; ++v)
-        {
-            // without a scale the product is stored as it is (an infinity
-            // would not pass y_scaled)
-            if constexpr (F32)
-                yr[v] = scaled ? y_scaled(acc[v], __int_as_float(__double2hiint(sxr[v])),
-                                          __int_as_float(__double2loint(sxr[v])))
-                               : acc[v];
-            else
-                yr[v] = acc[v] * sxr[v];
-        }
+            // without a scale the product is stored as it is
+            yr[v] = scaled ? y_scaled(acc[v], __int_as_float(__double2hiint(sxr[v])),
+                                      __int_as_float(__double2loint(sxr[v])))
+                           : acc[v];
         if (epi == 1)
         {
 #pragma unroll
             for (int v = 0; v < VEC; ++v)
-            {
-                if constexpr (F32)
-                    part[v] += f64_of_basis(xr[v]) * (static_cast<double>(yr[v]) * TWO_896);
-                else
-                    part[v] += xr[v] * yr[v];
-            }
+                part[v] += f64_of_finite(xr[v]) *
+                           (static_cast<double>(with_nan_of(xr[v], yr[v])) * TWO_896);
         }
         else if (epi == 2)
         {
 #pragma unroll
             for (int v = 0; v < VEC; ++v)
                 part[v] += static_cast<double>(yr[v]) * static_cast<double>(yr[v]);
+        }
+        else if (scaled)
+        {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) redo |= !(fabsf(yr[v]) <= FLT_MAX);
+        }
+    }
+    else if constexpr (PLAIN)
+    {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+        {
+            yr[v] = acc[v] * sxr[v];
+            if (epi == 1)
+                part[v] += xr[v] * yr[v];
+            else if (epi == 2)
+                part[v] += yr[v] * yr[v];
         }
     }
     else
@@ -463,6 +453,73 @@ __device__ __forceinline__ void finish_piece(const VT* acc, size_t o, int p0, co
         }
     }
     store_n<VT, VEC>(Y + o, yr);
+}
+
+// Whether a thread's LV columns, with their scales s and sums part, have to be
+// done again in FP64.  A NaN scale gives NaN there too.
+template <int LV, typename S>
+__device__ __forceinline__ bool needs_redo(bool redo, int epi, const double (&part)[LV], S scale)
+{
+    if (epi != 0)
+#pragma unroll
+        for (int v = 0; v < LV; ++v) redo |= !isfinite(part[v]) && !isnan(scale(v));
+    return redo;
+}
+
+// Four columns from p0 of a row of an FP32 product with scales, in FP64 as
+// k_spmm has them: `count` entries, entry u in column indices[u] with the
+// value vals[u * pitch]; the same sums in the same order.
+__device__ void redo_piece(const int32_t* __restrict__ indices,
+                           const float* __restrict__ vals, int pitch, int count,
+                           uint32_t row, int b, int p0, const float* X, const double* sx,
+                           float* Y, int epi, double* part)
+{
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int u = 0; u < count; ++u)
+    {
+        float x[4];
+        load_n<float, 4>(X + static_cast<size_t>(indices[u]) * b + p0, x);
+        const float a = vals[static_cast<size_t>(u) * pitch];
+        for (int v = 0; v < 4; ++v) acc[v] += a * x[v];
+    }
+    const size_t o = static_cast<size_t>(row) * b + p0;
+    for (int v = 0; v < 4; ++v)
+    {
+        const double s = sx ? sx[p0 + v] : 1.0;
+        const float y = static_cast<float>(static_cast<double>(acc[v]) * s);
+        const double ys = static_cast<double>(y);
+        if (epi == 1)
+            part[v] += static_cast<double>(X[o + v]) * ys;
+        else if (epi == 2)
+            part[v] += ys * ys;
+        Y[o + v] = y;
+    }
+}
+
+// The rows of a thread of k_spmm_rows again; its sums go to sums[probe].
+template <int LPR, int C>
+__noinline__ __device__ void redo_rows(const int32_t* __restrict__ indptr,
+                                       const int32_t* __restrict__ indices,
+                                       const float* __restrict__ vals, uint32_t nrows,
+                                       const float* X, const double* sx, float* Y, int epi,
+                                       double* sums)
+{
+    constexpr int RW = 32 / LPR;
+    constexpr int b = LPR * 4 * C;
+    const int lane = threadIdx.x & 31;
+    const uint32_t per_cta = (blockDim.x >> 5) * RW;
+    for (int p0 = lane % LPR * 4; p0 < b; p0 += LPR * 4)
+    {
+        double part[4] = {0.0, 0.0, 0.0, 0.0};
+        for (uint32_t r = blockIdx.x * per_cta + (threadIdx.x >> 5) * RW + lane / LPR; r < nrows;
+             r += gridDim.x * per_cta)
+        {
+            const int k = indptr[r];
+            redo_piece(indices + k, vals + k, 1, indptr[r + 1] - k, r, b, p0, X, sx, Y, epi, part);
+        }
+        if (epi != 0)
+            for (int v = 0; v < 4; ++v) sums[p0 + v] = part[v];
+    }
 }
 
 template <typename VT, int C>
@@ -506,6 +563,7 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
     }
 
     const VT* Xl = X + rl * VEC;
+    bool redo = false;
     // 32-bit rows (nrows < 2^31, and a stride more still fits)
     const uint32_t stride = gridDim.x * nwarps * RW;
     uint32_t row = (blockIdx.x * nwarps + warp) * RW + rs;
@@ -596,15 +654,20 @@ k_spmm_rows(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indi
             const int p0 = (q * LPR + rl) * VEC;
             finish_piece<VT, PLAIN>(acc + q * VEC, static_cast<size_t>(row) * b + p0, p0,
                                     sxr + q * VEC, sx != nullptr, shift, X, Y, Z, zc, zs, epi,
-                                    part + q * VEC);
+                                    part + q * VEC, redo);
         }
     }
 
-    if (epi == 0) return;
     // CTA reduction over warps and the rows of a warp, fixed order; then the
     // per-probe factor of the terms (s_p, 1 or zs_p)
+    if (epi != 0)
 #pragma unroll
-    for (int v = 0; v < LV; ++v) smem_rows[(warp * RW + rs) * b + probe(v)] = part[v];
+        for (int v = 0; v < LV; ++v) smem_rows[(warp * RW + rs) * b + probe(v)] = part[v];
+    if constexpr (PLAIN && sizeof(VT) == 4)
+        if (needs_redo(redo, epi, part, [&](int v) { return sx ? sx[probe(v)] : 1.0; }))
+            redo_rows<LPR, C>(indptr, indices, vals, nrows, X, sx, Y, epi,
+                              smem_rows + (warp * RW + rs) * b);
+    if (epi == 0) return;
     __syncthreads();
     for (int p = threadIdx.x; p < b; p += blockDim.x)
     {
@@ -2798,6 +2861,40 @@ struct RgShape {
     static constexpr int MINB = (RPW * 16 <= 64) ? 3 : 2;
 };
 
+// The items of a thread of k_spmm_rg again; its sums go to sums[probe].
+template <int LPR, int RPW>
+__noinline__ __device__ void redo_items(const int32_t* __restrict__ gptr,
+                                        const int32_t* __restrict__ gcol,
+                                        const float* __restrict__ gval, uint32_t nrows,
+                                        uint32_t ngroups, int G, int b, const float* X,
+                                        const double* sx, float* Y, int epi, double* sums)
+{
+    constexpr int RW = 32 / LPR;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t slices = static_cast<uint32_t>(b) / (4 * LPR);
+    const uint32_t parts = static_cast<uint32_t>(G) / RPW;
+    const uint32_t per_cta = (blockDim.x >> 5) / slices * RW;
+    const int p0 = static_cast<int>((warp & (slices - 1)) * LPR + lane % LPR) * 4;
+    double part[4] = {0.0, 0.0, 0.0, 0.0};
+    for (uint32_t i = blockIdx.x * per_cta + warp / slices * RW + lane / LPR; i < ngroups * parts;
+         i += gridDim.x * per_cta)
+    {
+        const int k = gptr[i / parts];
+        const int count = gptr[i / parts + 1] - k;
+        const uint32_t in_group = i % parts * RPW;
+        for (uint32_t r = 0; r < RPW; ++r)
+        {
+            const uint32_t row = i / parts * G + in_group + r;
+            if (row < nrows)
+                redo_piece(gcol + k, gval + static_cast<size_t>(k) * G + in_group + r, G, count,
+                           row, b, p0, X, sx, Y, epi, part);
+        }
+    }
+    if (epi != 0)
+        for (int v = 0; v < 4; ++v) sums[p0 + v] = part[v];
+}
+
 template <typename VT, int LPR, int RPW, bool PLAIN>
 __global__ void __launch_bounds__(256, RgShape<VT, RPW>::MINB)
 k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
@@ -2830,6 +2927,7 @@ k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
     }
 
     const VT* Xl = X + p0;
+    bool redo = false;
     const uint32_t items = ngroups * parts;
     const uint32_t per_cta = static_cast<uint32_t>(nwarps) / slices * RW;
     const uint32_t stride = gridDim.x * per_cta;
@@ -2902,15 +3000,19 @@ k_spmm_rg(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
         for (int r = 0; r < RPW; ++r)
             if (row0 + r < nrows)
                 finish_piece<VT, PLAIN>(acc[r], static_cast<size_t>(row0 + r) * b + p0, p0, sxr,
-                                        sx != nullptr, shift, X, Y, Z, zc, zs, epi, part);
+                                        sx != nullptr, shift, X, Y, Z, zc, zs, epi, part,
+                                        redo);
     }
 
-    if (epi == 0) return;
     // fixed order: the CTA's warps of a slice, the items of a warp
+    double* sums = smem_rg + static_cast<size_t>(static_cast<uint32_t>(warp) / slices * RW + rs) * b;
+    if (epi != 0)
 #pragma unroll
-    for (int v = 0; v < VEC; ++v)
-        smem_rg[static_cast<size_t>(static_cast<uint32_t>(warp) / slices * RW + rs) * b + p0 + v] =
-            part[v];
+        for (int v = 0; v < VEC; ++v) sums[p0 + v] = part[v];
+    if constexpr (PLAIN && sizeof(VT) == 4)
+        if (needs_redo(redo, epi, part, [&](int v) { return sx ? sx[p0 + v] : 1.0; }))
+            redo_items<LPR, RPW>(gptr, gcol, gval, nrows, ngroups, G, b, X, sx, Y, epi, sums);
+    if (epi == 0) return;
     __syncthreads();
     for (int p = threadIdx.x; p < b; p += blockDim.x)
     {
