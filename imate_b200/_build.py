@@ -17,7 +17,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 SOURCES = ["slq_engine.cu", "slq_mlp.cu", "slq_rng.cpp", "slq_stats.cpp",
            "slq_order.cpp"]
 HEADERS = ["slq_kernels.cuh", "slq_blk.cuh", "slq_once.h", "slq_ql.cuh",
-           "slq_rng.h", "slq_scale.cuh", "slq_tc.cuh"]
+           "slq_rng.h", "slq_rule.h", "slq_scale.cuh", "slq_tc.cuh"]
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -32,6 +32,7 @@
 #include "slq_kernels.cuh"
 #include "slq_once.h"
 #include "slq_rng.h"
+#include "slq_rule.h"
 
 using namespace slq;
 
@@ -1599,6 +1600,42 @@ slq_status spmm_rg(Launcher& L, int rpw, const int32_t* gptr, const int32_t* gco
     return fail(SLQ_ERR_BAD_ARG, "row-group SpMM: unsupported tile");
 }
 
+// Whole groups per warp (k_spmm_rgs): b = 32 or 64, groups of 4 or 8 rows.
+template <typename VT, int LV, int G>
+slq_status spmm_rgs_inst(Launcher& L, const int32_t* gptr, const int32_t* gcol, const VT* gval,
+                         int64_t nrows, const VT* X, const double* sx, double shift, VT* Y,
+                         const VT* Z, const double* zc, const double* zs, int epi,
+                         double* partials, int64_t nnz, int64_t xrows, int* grid_out)
+{
+    ProfScope prof(SLQ_K_SPMM, spmm_bytes<VT>(nnz, nrows, xrows, 32 * LV, Z != nullptr), L.st);
+    const int64_t ng = (nrows + G - 1) / G;
+    const int grid =
+        static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((ng + 7) / 8, int64_t(L.sms) * 4)));
+    SLQ_TRY(launch_pdl(L, k_spmm_rgs<VT, LV, G>, grid, 256, 0, gptr, gcol, gval, nrows, ng, X, sx,
+                       shift, Y, Z, zc, zs, epi, partials));
+    ++L.launches;
+    *grid_out = grid;
+    return SLQ_OK;
+}
+
+template <typename VT>
+slq_status spmm_rgs(Launcher& L, const int32_t* gptr, const int32_t* gcol, const VT* gval,
+                    int64_t nrows, int G, int b, const VT* X, const double* sx, double shift,
+                    VT* Y, const VT* Z, const double* zc, const double* zs, int epi,
+                    double* partials, int64_t nnz, int64_t xrows, int* grid_out)
+{
+#define SLQ_RGS_CASE(LV, GG)                                                                   \
+    if (b == 32 * LV && G == GG)                                                               \
+        return spmm_rgs_inst<VT, LV, GG>(L, gptr, gcol, gval, nrows, X, sx, shift, Y, Z, zc,   \
+                                         zs, epi, partials, nnz, xrows, grid_out);
+    SLQ_RGS_CASE(1, 4)
+    SLQ_RGS_CASE(1, 8)
+    SLQ_RGS_CASE(2, 4)
+    SLQ_RGS_CASE(2, 8)
+#undef SLQ_RGS_CASE
+    return fail(SLQ_ERR_BAD_ARG, "row-group SpMM: unsupported tile");
+}
+
 // Tensor-core row-group SpMM (k_spmm_tc): 16-row groups, b = 128 NS, two
 // CTAs per SM; X rows by TMA gathers (xmap as for k_spmm_rgt).
 template <int NS>
@@ -1716,11 +1753,10 @@ slq_status spmm_blk_inst(Launcher& L, const slq_op* op, int transpose, int b, co
 // (FP32, G = 8, b = 128 or 256), row-group with the widest LV <= 4, CSR.
 // ---------------------------------------------------------------------------
 
-enum { CAND_CSR = 0, CAND_RG = 1, CAND_TMA = 2, CAND_TC = 3, CAND_BLK = 4 };
 
 struct SpmmCand {
     int kind, g, lv, ns;
-    int rpw = 0;  // CAND_RG: rows of the group per warp
+    int rpw = 0;  // CAND_RG: rows of the group per warp, 0 whole groups (k_spmm_rgs)
 };
 
 template <typename VT>
@@ -1740,6 +1776,7 @@ int spmm_candidates(const slq_op* op, int transpose, int b, SpmmCand* out)
     if (b >= 32 && (sizeof(VT) == 4 || G <= 8))
         for (int rpw = 4; rpw <= std::min(G, 8); rpw *= 2)
             out[n++] = {CAND_RG, G, vec, std::max(1, G / rpw * b / (32 * vec)), rpw};
+    if ((b == 32 || b == 64) && G <= 8) out[n++] = {CAND_RG, G, b / 32, 1, 0};
     if (sizeof(VT) == 4 && (G == 8 || G == 16) && (b == 128 || b == 256))
         out[n++] = {CAND_TMA, G, 4, b / 128};
     if (sizeof(VT) == 4 && G == 16 && (b == 128 || b == 256))
@@ -1806,6 +1843,9 @@ slq_status spmm_cand(Launcher& L, const slq_op* op, int transpose, const SpmmCan
     {
         const VT* gval = static_cast<const VT*>(transpose ? op->t_gval : op->a_gval);
         constexpr int VEC = 16 / static_cast<int>(sizeof(VT));
+        if (c.rpw == 0)
+            return spmm_rgs<VT>(L, gptr, gcol, gval, rows, c.g, b, X, sx, shift, Y, Z, zc, zs, epi,
+                                partials, op->nnz, xrows, grid_out);
         if (b >= 32 * VEC)
             return spmm_rg<VT, 32>(L, c.rpw, gptr, gcol, gval, rows, c.g, b, X, sx, shift, Y, Z, zc,
                                    zs, epi, partials, op->nnz, xrows, grid_out);
@@ -1829,41 +1869,6 @@ int log2_width(int b)
     int lg = 0;
     while ((1 << lg) < b) ++lg;
     return lg;
-}
-
-// The product of an operator without a block format and without a tuned
-// choice: CSR or row groups (rpw rows of a group per warp) or their TMA form,
-// by rows, group width and block width.  Measured on correlation matrices
-// with L2 flushed between products, as the passes over the basis leave it, us
-// (CSR / row groups; TMA after a slash of its own):
-//   FP32, 8-row groups   n 8,000 b 64: 14 / 47, b 256: 29 / 53; n 16,400 b 64:
-//                        27 / 27, b 128: 35 / 31; n 30,011 b 256: 64 / 62; n
-//                        65,537 b 64: 74 / 70, b 128: 113 / 94 / 90, b 256:
-//                        181 / 154 / 164; n 150,000 b 128: 135 / 127 / 137
-//   FP32, 16-row groups  n 32,768 b 64: 61 / 104, b 256: 152 / 197 / 198; n
-//                        50,000 b 256: 275 / 294 / 256; n 100,003 b 64: 152 /
-//                        172, b 128: 246 / 244 / 219, b 256: 398 / 423 / 342;
-//                        n 262,144 b 32: 459 / 401, b 64: 793 / 557, b 128:
-//                        1,214 / 895 / 682
-//   FP64, 8-row groups   n 17,000 b 64: 35 / 37; n 40,009 b 64: 80 / 98; n
-//                        100,000 b 32: 88 / 107, b 64: 133 / 146
-// Small matrices have too few groups to hide a gather's latency, and FP64
-// groups lose by their padding at every size.
-struct SpmmRule {
-    int kind, rpw;
-};
-
-template <typename VT>
-SpmmRule spmm_rule(int64_t rows, int G, int b)
-{
-    const SpmmRule csr{CAND_CSR, 0}, groups{CAND_RG, std::min(G, 8)};
-    if (sizeof(VT) == 8 || !G || rows < 16384 || b < 32 || b > 256) return csr;
-    if (G == 16)
-    {
-        if (b >= 128) return rows >= (b == 128 ? 65536 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
-        return rows >= 200000 ? groups : csr;
-    }
-    return (b >= 128 || rows >= 65536) ? groups : csr;
 }
 
 // Operator product on a block.  An autotuned choice (slq_operator_tune /
@@ -1907,7 +1912,8 @@ slq_status op_spmm(Launcher& L, const slq_op* op, int transpose, int b, const VT
         if (cands[i].kind == CAND_BLK && have_blk) pick = i;
     if (cands[pick].kind != CAND_BLK)
     {
-        const SpmmRule want = spmm_rule<VT>(rows, op->group_rows, b);
+        const SpmmRule want = spmm_rule(sizeof(VT) == 8, rows, double(op->nnz) / double(rows),
+                                        op->group_rows, b);
         for (int i = 0; i < nc; ++i)
             if (usable(cands[i]) && cands[i].kind == want.kind &&
                 (want.kind != CAND_RG || cands[i].rpw == want.rpw))

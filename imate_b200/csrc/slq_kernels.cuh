@@ -2843,6 +2843,128 @@ __global__ void k_rg_fill(const int32_t* __restrict__ ptr, const int32_t* __rest
     }
 }
 
+// Blocks of b = 32 LV probes, whole groups per warp: a lane owns LV probes of all
+// G rows, 32 union columns and their values are staged in shared memory at a
+// time, and two gathers are in flight.  Every value is read from memory once
+// per group, where the parts below read it once per part and lane; with few
+// probes that is most of the traffic, and with LV x G accumulators of at most
+// 16 doubles a warp keeps enough in flight.  Figures beside spmm_rule.
+template <typename VT, int LV, int G>
+__global__ void __launch_bounds__(256, 2)
+k_spmm_rgs(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gcol,
+           const VT* __restrict__ gval, int64_t nrows, int64_t ngroups, const VT* X,
+           const double* sx, double shift, VT* __restrict__ Y, const VT* Z, const double* zc,
+           const double* zs, int epi, double* __restrict__ partials)
+{
+    constexpr int b = 32 * LV;
+    __shared__ int32_t s_col[8][32];
+    __shared__ __align__(16) VT s_val[8][32][G];
+    __shared__ double s_red[8][b];
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int p0 = lane * LV;
+
+    double sxr[LV], zcr[LV], part[LV];
+#pragma unroll
+    for (int v = 0; v < LV; ++v)
+    {
+        sxr[v] = sx ? sx[p0 + v] : 1.0;
+        zcr[v] = Z ? zc[p0 + v] * zs[p0 + v] : 0.0;
+        part[v] = 0.0;
+    }
+
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * 8;
+    for (int64_t g = static_cast<int64_t>(blockIdx.x) * 8 + warp; g < ngroups; g += stride)
+    {
+        VT acc[G][LV];
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+#pragma unroll
+            for (int v = 0; v < LV; ++v) acc[r][v] = VT(0);
+        const int u0 = __ldg(gptr + g);
+        const int u1 = __ldg(gptr + g + 1);
+        for (int base = u0; base < u1; base += 32)
+        {
+            const int cnt = min(32, u1 - base);
+            if (lane < cnt)
+            {
+                s_col[warp][lane] = __ldg(gcol + base + lane);
+                VT tmp[G];
+                ldg_n<VT, G>(gval + static_cast<int64_t>(base + lane) * G, tmp);
+                store_n<VT, G>(&s_val[warp][lane][0], tmp);
+            }
+            __syncwarp();
+            int t = 0;
+            for (; t + 2 <= cnt; t += 2)
+            {
+                VT x0[LV], x1[LV], a0[G], a1[G];
+                load_n<VT, LV>(X + static_cast<int64_t>(s_col[warp][t]) * b + p0, x0);
+                load_n<VT, LV>(X + static_cast<int64_t>(s_col[warp][t + 1]) * b + p0, x1);
+                load_n<VT, G>(&s_val[warp][t][0], a0);
+                load_n<VT, G>(&s_val[warp][t + 1][0], a1);
+#pragma unroll
+                for (int r = 0; r < G; ++r)
+#pragma unroll
+                    for (int v = 0; v < LV; ++v)
+                    {
+                        acc[r][v] += a0[r] * x0[v];
+                        acc[r][v] += a1[r] * x1[v];
+                    }
+            }
+            if (t < cnt)
+            {
+                VT x0[LV], a0[G];
+                load_n<VT, LV>(X + static_cast<int64_t>(s_col[warp][t]) * b + p0, x0);
+                load_n<VT, G>(&s_val[warp][t][0], a0);
+#pragma unroll
+                for (int r = 0; r < G; ++r)
+#pragma unroll
+                    for (int v = 0; v < LV; ++v) acc[r][v] += a0[r] * x0[v];
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+        {
+            const int64_t row = g * G + r;
+            if (row >= nrows) break;
+            const int64_t o = row * b + p0;
+            VT xr[LV], zr[LV], yr[LV];
+            if (shift != 0.0 || epi == 1) load_n<VT, LV>(X + o, xr);
+            if (Z) load_n<VT, LV>(Z + o, zr);
+#pragma unroll
+            for (int v = 0; v < LV; ++v)
+            {
+                double y = static_cast<double>(acc[r][v]) * sxr[v];
+                if (shift != 0.0) y += shift * (sxr[v] * static_cast<double>(xr[v]));
+                if (Z) y -= zcr[v] * static_cast<double>(zr[v]);
+                yr[v] = static_cast<VT>(y);
+                const double ys = static_cast<double>(yr[v]);
+                if (epi == 1)
+                    part[v] += (sxr[v] * static_cast<double>(xr[v])) * ys;
+                else if (epi == 2)
+                    part[v] += ys * ys;
+                else if (epi == 3)
+                    part[v] += (zs[p0 + v] * static_cast<double>(zr[v])) * ys;
+            }
+            store_n<VT, LV>(Y + o, yr);
+        }
+    }
+
+    if (epi == 0) return;
+#pragma unroll
+    for (int v = 0; v < LV; ++v) s_red[warp][p0 + v] = part[v];
+    __syncthreads();
+    for (int p = threadIdx.x; p < b; p += blockDim.x)
+    {
+        double s = 0.0;
+        for (int w = 0; w < 8; ++w) s += s_red[w][p];
+        partials[static_cast<int64_t>(blockIdx.x) * b + p] = s;
+    }
+}
+
 // One item is RPW of a group's G rows times the 16-byte pieces of LPR lanes:
 // the G / RPW parts of a group and the NS = b / (VEC LPR) slices of its probes
 // go to neighbouring warps, which gather the same X rows from L1 (LPR < 32:

@@ -375,9 +375,11 @@ slq_status slq_run(slq_op* op, const slq_params* p, const double* parameters,
  * block width are the storage formats the operator holds crossed with their
  * tiles: CSR; row-group (the operator's group_rows rows sharing a union of
  * columns; float64: at most 8 rows) from 32 probes on, a lane holding 16
- * bytes of probes and a warp 4 or 8 of the group's rows; in FP32 with 8- or 16-row groups at b = 128 or 256, the
- * row-group kernel whose X rows arrive by TMA gathers; and in FP32 with
- * 16-row groups at b = 128 or 256, the tensor-core row-group kernel
+ * bytes of probes and a warp 4 or 8 of the group's rows, and at 32 and 64
+ * probes whole groups of 4 or 8 rows per warp (slices 1); in FP32 with 8- or
+ * 16-row groups at b = 128 or 256, the row-group kernel whose X rows arrive
+ * by TMA gathers; and in FP32 with 16-row groups at b = 128 or 256, the
+ * tensor-core row-group kernel
  * (tcgen05 kind::tf32 on TF32 hi/lo splits of both operands, accumulators
  * in tensor memory; FP32-level accuracy, chosen only by the tuner or
  * slq_operator_set_variant).  slq_operator_tune times every candidate (reps
