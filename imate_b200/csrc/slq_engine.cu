@@ -1913,7 +1913,7 @@ slq_status op_spmm(Launcher& L, const slq_op* op, int transpose, int b, const VT
     if (cands[pick].kind != CAND_BLK)
     {
         const SpmmRule want = spmm_rule(sizeof(VT) == 8, rows, double(op->nnz) / double(rows),
-                                        op->group_rows, b);
+                                        op->group_rows, b, have_row);
         for (int i = 0; i < nc; ++i)
             if (usable(cands[i]) && cands[i].kind == want.kind &&
                 (want.kind != CAND_RG || cands[i].rpw == want.rpw))

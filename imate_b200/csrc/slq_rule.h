@@ -21,7 +21,9 @@ struct SpmmRule {
 // The product of an operator without a block format and without a tuned
 // choice, by rows, entries per row, group width (0: no groups) and block
 // width: CSR, parts of row groups, whole row groups (b = 32 or 64, groups of 4
-// or 8) or the TMA form (b = 128 or 256, groups of 16).  Measured on
+// or 8) or the TMA form (b = 128 or 256, groups of 16; only with a tensor map
+// of the probe block, which slq_operator_dot and the second product of the
+// normal equations do not have).  Measured on
 // correlation matrices inside Krylov runs, whose passes over the basis leave
 // L2 to the basis, us per product (n x entries per row, b: CSR / parts / whole
 // groups):
@@ -46,8 +48,12 @@ struct SpmmRule {
 //                 65,537 x 60, 128: 121 / 120 / 133, 256: 208 / 214 / 198;
 //                 80,000 x 99, 128: 222 / 238 / 205;  150,000 x 60, 128: 253 /
 //                 265 / 237;  220,000 x 60, 32: 136 / 151, 64: 234 / 215
+//   the same, no tensor map  100,003 x 90, 256: 432 / 404;  150,000 x 31, 256:
+//                 227 / 288;  220,000 x 61, 128: 354 / 322, 256: 748 / 626;
+//                 262,144 x 149, 128: 1,124 / 748, 256: 2,487 / 1,408
 // Small matrices have too few groups to hide a gather's latency.
-inline SpmmRule spmm_rule(bool f64, int64_t rows, double per_row, int G, int b)
+inline SpmmRule spmm_rule(bool f64, int64_t rows, double per_row, int G, int b,
+                          bool have_map)
 {
     const SpmmRule csr{CAND_CSR, 0}, parts{CAND_RG, std::min(G, 8)}, whole{CAND_RG, 0};
     if (!G || rows < 16384 || b < 32 || b > 256) return csr;
@@ -59,7 +65,8 @@ inline SpmmRule spmm_rule(bool f64, int64_t rows, double per_row, int G, int b)
     }
     if (G == 16)
     {
-        if (b >= 128) return rows >= (b == 128 ? 65536 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
+        if (b >= 128 && have_map)
+            return rows >= (b == 128 ? 65536 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
         return rows >= 200000 ? parts : csr;
     }
     if (b == 32 && long_rows && rows < (G == 4 ? 98304 : 65536)) return whole;

@@ -15,10 +15,10 @@ CSR, GROUPS, TMA = 0, 1, 2
 def rule(tmp_path_factory):
     lib = native.load("rule", tmp_path_factory.mktemp("rule"))
 
-    def pick(f64, rows, per_row, G, b):
+    def pick(f64, rows, per_row, G, b, have_map=True):
         out = (ctypes.c_int * 2)()
         lib.rule(int(f64), ctypes.c_longlong(rows), ctypes.c_double(per_row),
-                 G, b, out)
+                 G, b, int(have_map), out)
         return tuple(out)
     return pick
 
@@ -31,6 +31,7 @@ def test_choices_exist_for_the_operator(rule, f64, G):
                      200000, 2000000):
             for per_row in (0.0, 8.0, 48.0, 500.0):
                 kind, rpw = rule(f64, rows, per_row, G, b)
+                assert rule(f64, rows, per_row, G, b, False)[0] != TMA
                 if kind == CSR:
                     continue
                 assert G and b >= 32
@@ -62,3 +63,12 @@ def test_choices_exist_for_the_operator(rule, f64, G):
 ])
 def test_measured_choices(rule, f64, rows, per_row, G, b, want):
     assert rule(f64, rows, per_row, G, b) == want
+
+
+@pytest.mark.parametrize("rows,b,want", [
+    # parts where the TMA form has no map: 748 us against 1,124, 626 against
+    # 748; CSR below: 227 against 288
+    (262144, 128, (GROUPS, 8)), (262144, 256, (GROUPS, 8)),
+    (220000, 256, (GROUPS, 8)), (150000, 256, (CSR, 0))])
+def test_choice_without_a_tensor_map(rule, rows, b, want):
+    assert rule(False, rows, 60.0, 16, b, False) == want
