@@ -66,7 +66,7 @@ inline SpmmRule spmm_rule(bool f64, int64_t rows, double per_row, int G, int b,
     if (G == 16)
     {
         if (b >= 128 && have_map)
-            return rows >= (b == 128 ? 65536 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
+            return rows >= (b == 128 ? 73728 : 49152) ? SpmmRule{CAND_TMA, 0} : csr;
         return rows >= 200000 ? parts : csr;
     }
     if (b == 32 && long_rows && rows < (G == 4 ? 98304 : 65536)) return whole;

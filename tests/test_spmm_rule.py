@@ -58,6 +58,8 @@ def test_choices_exist_for_the_operator(rule, f64, G):
     (False, 8000, 30.3, 8, 256, (CSR, 0)),
     # parts: 152 against 208
     (False, 65537, 60.1, 8, 256, (GROUPS, 8)),
+    # CSR: 121 against 133 (TMA)
+    (False, 65537, 60.1, 16, 128, (CSR, 0)),
     # TMA: 205 against 222
     (False, 80000, 99.3, 16, 128, (TMA, 0)),
 ])
