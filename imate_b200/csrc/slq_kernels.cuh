@@ -2070,17 +2070,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) k_stream(const StreamArgs<V
                     if (++s == a.S) { s = 0; phase ^= 1; }
                 }
             }
-            if (!ok)
-            {
-                // let the copies already issued land before the CTA leaves
-                int s2 = 0;
-                uint32_t ph2 = 0;
-                for (int64_t k = 0; k < issued; ++k)
-                {
-                    if (k + a.S >= issued) mbar_wait(&full[s2], ph2, abort_flag + 1);
-                    if (++s2 == a.S) { s2 = 0; ph2 ^= 1; }
-                }
-            }
+            // the copies in flight land before the CTA leaves: the consumers may
+            // have given up after the last one was issued
+            for (int64_t k = max(int64_t(0), issued - a.S); k < issued; ++k)
+                mbar_wait(&full[k % a.S], static_cast<uint32_t>((k / a.S) & 1), abort_flag + 1);
         }
     }
     else
