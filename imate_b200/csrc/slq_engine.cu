@@ -92,7 +92,7 @@ struct Carver {
 
 int g_num_sms = 0;
 
-// test hook (slq_debug_fail_stream_waits): streaming launches left whose
+// test hook (slq_debug_fail_stream_waits): passes over the basis left whose
 // first wait is to run out at once
 std::atomic<int> g_fail_stream_waits{0};
 // test hook (slq_debug_blocks_sorted_keys): build block unions by sorting
@@ -1994,7 +1994,13 @@ slq_status stream_pass(Launcher& L, int64_t n, int b, const VT* W, VT* Wout, int
     a.x16 = x16;
     a.x16exp = x16exp;
     if (g_fail_stream_waits.load() > 0 && g_fail_stream_waits.fetch_sub(1) > 0)
-        a.fail_first_wait = 1;
+    {
+        // a pass that has no waits leaves what a wait that ran out would
+        if (MODE == 0 && !loads)
+            a.fail_first_wait = 1;
+        else
+            SLQ_CK(cudaMemsetAsync(error, 1, sizeof(int32_t), L.st));
+    }
     // one CTA per SM; the three-term update takes all probes of a row together.
     // No more CTAs than 16-byte pieces for all threads: every CTA is a row of
     // partial sums to add.

@@ -1957,7 +1957,7 @@ struct StreamArgs {
     int want_norm;
     double* partials;     // dots: [grid.x][J][b]; reorth: [grid.x][b]
     int32_t* error;       // set to 1 when a wait runs out
-    int fail_first_wait;  // test hook: the consumers' first wait runs out at once
+    int fail_first_wait;  // test hook (k_stream): the consumers' first wait runs out at once
     // the block SpMM's split probe block, written by the pass that writes the
     // next Krylov vector (float only): dots with do_update write the partial
     // sums of |w|^2 of the updated w, [grid.x][b] (wn2_out); the last reorth
@@ -2373,11 +2373,6 @@ k_three_term(const StreamArgs<VT> a)
     const int b = a.b;
     pdl_wait();
     pdl_trigger();
-    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
-    {
-        if (tid == 0) atomicExch(a.error, 1);
-        return;
-    }
     double cj[VEC], cm[VEC], nacc[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; ++i)
@@ -2472,11 +2467,6 @@ __global__ void __launch_bounds__(REORTH_THREADS, 1) k_reorth(const StreamArgs<V
     const int p0 = blockIdx.y * PT;
     pdl_wait();
     pdl_trigger();
-    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
-    {
-        if (tid == 0) atomicExch(a.error, 1);
-        return;
-    }
     double nacc[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; ++i) nacc[i] = 0.0;
@@ -2663,11 +2653,6 @@ __global__ void __launch_bounds__(DOTS_THREADS, 1) k_dots(const StreamArgs<doubl
     for (int i = 0; i < J; ++i) acc[i * DOTS_THREADS] = 0.0;
     pdl_wait();
     pdl_trigger();
-    if (a.fail_first_wait)  // test hook: as a streaming pass whose wait ran out
-    {
-        if (tid == 0) atomicExch(a.error, 1);
-        return;
-    }
     double cj = 0.0, cm = 0.0;
     if (upd)
     {

@@ -604,12 +604,14 @@ slq_status slq_device_info(int* num_devices, int* num_sms,
 const char* slq_last_error(void);
 int slq_abi_version(void);
 
-/* Test hook (no counterpart in the reference): the next `count` launches of
- * the streaming update / reorthogonalisation kernel treat their first
- * mbarrier wait as timed out.  That wait then takes the path of a real one
- * that ran out -- the CTA sets the run's error word, stops, waits (with the
- * full bound) for the copies it issued, and the call returns
- * SLQ_ERR_TIMEOUT -- so the failure path can be exercised without a fault.
+/* Test hook (no counterpart in the reference): the next `count` passes over
+ * the Krylov basis report a wait that ran out, and the call returns
+ * SLQ_ERR_TIMEOUT, so that the failure path can be exercised without a fault.
+ * In the streaming kernel (float32 inner products, and float64 ones of more
+ * than 48 vectors) the first mbarrier wait takes the path of a real one: the
+ * CTA sets the run's error word, stops, and waits (with the full bound) for
+ * the copies it issued.  The other passes have no waits; for them the host
+ * sets the error word.
  * 0 switches it off. */
 slq_status slq_debug_fail_stream_waits(int count);
 
