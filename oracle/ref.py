@@ -32,6 +32,11 @@ _lib = None
 _gpu_lib = None
 
 
+class NotBuilt(FileNotFoundError):
+    """A reference library that was not built: its sources are not part of
+    this repository."""
+
+
 def _capsule_pointer(capsule):
     get_name = ctypes.pythonapi.PyCapsule_GetName
     get_name.restype = ctypes.c_char_p
@@ -63,7 +68,7 @@ def load():
     if _lib is not None:
         return _lib
     if not available():
-        raise FileNotFoundError(
+        raise NotBuilt(
             "reference CPU library not built: run `make -C oracle ref` "
             "where the reference sources are present")
     lib = ctypes.CDLL(REF_SO)
@@ -84,7 +89,7 @@ def load_gpu():
     if _gpu_lib is not None:
         return _gpu_lib
     if not gpu_available():
-        raise FileNotFoundError(
+        raise NotBuilt(
             "reference GPU library not built: run `make -C oracle ref_gpu` "
             "where the reference sources are present")
     lib = ctypes.CDLL(REF_GPU_SO)
