@@ -3803,16 +3803,19 @@ k_spmm_tc(const __grid_constant__ CUtensorMap xmap, const int32_t* __restrict__ 
 //
 // Y[M][b] = A[M][K] X[K][b] for a dense row-major A.  Each operand is split
 // into three BF16 parts, h = rn_bf16(v), m = rn_bf16(v - h) and l = v - h - m,
-// which hold all 24 bits and FP32's range.  The parts of A are made once,
-// [part][row][k] with a row pitch ldk (a multiple of 32, zero-padded); each
-// product splits and transposes the probe block likewise (XT[part][p][k], k
-// contiguous), at most 256 probes at a time.
+// which hold all 24 bits from 2^-109 to FP32's largest value.  (Below, l runs
+// into BF16's subnormals: an error of 6e-7 of |A| |X| with entries of 2^-116 and
+// 1e-5 of 2^-120, where the TF32 pairs had 3e-7 and 1.3e-6.  FP32 Krylov runs do
+// not get there: the products of two such entries vanish.)  The parts of A are
+// made once, [part][row][k] with a row pitch ldk (a multiple of 32,
+// zero-padded); each product splits and transposes the probe block likewise
+// (XT[part][p][k], k contiguous), at most 256 probes at a time.
 //
 // A CTA computes 128-row tiles of Y (persistent over the tiles): TMA loads
 // 32-value K slices of A's and XT's parts (64-byte rows, SWIZZLE_64B; one
 // copy brings all three parts) into a ring, one thread issues per K step of
 // 16 the six kind::f16 MMAs l h + m m + h l + m h + h m + h h (the terms
-// left out are below 2^-24) into an FP32 accumulator in tensor memory
+// left out are below 2^-22) into an FP32 accumulator in tensor memory
 // (D[128][N], lane = row, column = probe).  The tensor core's FP32
 // accumulation does not round to nearest: its error is biased towards zero
 // and grows with the number of MMAs into one accumulator.  So each 64-value K

@@ -66,6 +66,25 @@ def test_the_bound_needs_every_product():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("a_scale,x_scale", [(2.0**-100, 1.0), (1.0, 2.0**-100),
+                                             (2.0**60, 2.0**-108),
+                                             (2.0**-108, 2.0**60),
+                                             (2.0**63, 2.0**62)])
+def test_scales_far_from_one(cuda, a_scale, x_scale):
+    # l is at least 2^-24 of a value: 2^-132, one of BF16's subnormals; sums of
+    # the smallest products below 2^-126 may be lost, 3 * 2^-126 of 2^-100
+    import torch
+    rng = np.random.default_rng(3)
+    a = _values(rng, 150)
+    X = _values(rng, 150 * 40).reshape(150, 40)
+    A = np.diag(a * np.float32(a_scale))
+    op = ib.Matrix(A).get_device_operator()
+    Y = op.dot(torch.from_numpy(X * np.float32(x_scale)).cuda()).cpu().numpy()
+    want = a[:, None].astype(np.float64) * X * (a_scale * x_scale)
+    assert np.max(np.abs(Y - want) / np.abs(want)) <= BOUND
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols,width", [
     (130, 1, 48), (300, 200, 16), (129, 97, 256), (9700, 64, 33),
     (70, 2100, 300)])
