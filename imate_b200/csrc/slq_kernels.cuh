@@ -347,7 +347,11 @@ k_spmm(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
 // 340 with a branch for every piece instead of redo_rows); 89,999 rows of 5, b = 128, FP64: 102 -> 56; 16,384 rows of
 // 2, b = 256, FP64, both directions: 58 -> 33; a 524,288 x 131,072 matrix
 // with 16 random entries per column, b = 128, FP32, mean of A and A^T:
-// 216 -> 172.
+// 216 -> 172.  Rows of 2 / 5 / 7 / 9 / 14 / 20 entries, before and now: 524,176
+// rows, b = 256, FP32: 471, 576, 639, 690, 859, 1,202 -> 266, 303, 395, 422, 510,
+// 586; 100,000 rows, b = 64, FP32: 42, 49, 53, 53, 65, 72 -> 26, 26, 27, 31, 33,
+// 43; 89,999 rows, b = 128, FP64: 86, 102, 110, 113, 148, 169 -> 45, 51, 61, 64,
+// 79, 97.
 // ---------------------------------------------------------------------------
 
 // L2 prefetch of [p, p + bytes) by n lanes (lane 0 .. n - 1), a 128-byte line
@@ -525,8 +529,9 @@ __noinline__ __device__ void redo_rows(const int32_t* __restrict__ indptr,
 template <typename VT, int C>
 struct SpmmRowsShape {
     // entries gathered at once and resident 256-thread blocks per SM: swept
-    // at the sizes above (FP32 C = 2: 5 entries at 3 blocks, 8 at 2 and 4 at 4
-    // were 10 to 40 % slower; C = 1: 8 at 4 best)
+    // on rows of 5 entries (FP32 C = 2: 5 entries at 3 blocks, 8 at 2 and 4 at 4
+    // were 10 to 40 % slower; C = 1: 8 at 4 best); a remainder costs a batch of
+    // predicated loads, and no length from 2 to 20 is behind the kernel before
     static constexpr int U = C == 1 ? 8 : C == 2 ? 5 : C == 4 ? 3 : 2;
     static constexpr int MINB = C == 1 ? 4 : C == 2 ? 3 : C == 4 ? 2 : 1;
 };
