@@ -26,12 +26,16 @@ __device__ __forceinline__ void scale_pair(double s, float& hi, float& lo)
 // is, where that does not hold: results next to FP32's largest value or past
 // it, results below 2^-100 (whose remainder may be below the subnormals), an x
 // that is not finite and a scale without a pair.  The caller looks for these
-// and computes them in FP64.
+// and computes them in FP64.  A zero product is taken as it is: of an x or of
+// the scale of a stopped probe that is zero, or below 2^-150.
 __device__ __forceinline__ float y_scaled(float x, float hi, float lo)
 {
     const float p = x * hi;
     const float y = p + fmaf(x, lo, fmaf(x, hi, -p));
-    return fabsf(p) < 0x1p-100f && x != 0.0f ? __int_as_float(0x7fc00000) : y;
+    // 0 < |p| < 2^-100, from the bits without the sign; a zero passes
+    constexpr unsigned SMALL = 2u * 0x0d800000u;
+    const bool small = 2u * static_cast<unsigned>(__float_as_int(p)) - 1u < SMALL - 1u;
+    return small ? __int_as_float(0x7fc00000) : y;
 }
 
 // 2^-896 x as a double, from the bits of x: exact for every finite x, zeros

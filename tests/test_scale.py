@@ -77,3 +77,10 @@ def test_ordinary_values_and_zeros_need_no_second_product(scale):
     x[::3] = 0.0
     _, wide, _ = scale(x, np.full(x.size, 0.0123456789))
     assert not np.any(wide)
+
+
+def test_a_stopped_probe_needs_no_second_product(scale):
+    # its scale is zero, its vector is not
+    x = np.random.default_rng(3).standard_normal(1000).astype(np.float32)
+    y, wide, _ = scale(x, np.zeros(x.size))
+    assert not np.any(wide) and not np.any(y)
